@@ -22,6 +22,7 @@
 #include "fdtd3d_adjoint.cuh"
 #include "fdtd3d_kernels.cuh"
 #include "learned_band.cuh"
+#include "sweep_registry.h"
 #include "tb_registry.h"
 #include "tma_registry.h"
 #include "viz_kernels.cuh"
@@ -205,10 +206,15 @@ int encode_map(CUtensorMap* m, const float* base, int nx, int ny, int nz, int bz
 // TMA kernel registry
 // ---------------------------------------------------------------------------
 
-// autotune results: (nx, ny, nz, mode, cbarr) -> (cfg index, x_chunk, axis split,
-// blocked cfg index or -1, blocked x_chunk)
+// autotune results: (nx, ny, nz, mode, cbarr) -> one-step launch shape (cfg
+// index, x_chunk, axis split), blocked shape (cfg index or -1, x_chunk), and
+// whether in-place sweeps beat both
 std::mutex g_tune_mu;
-std::map<std::tuple<int, int, int, int, int>, std::tuple<int, int, int, int, int>> g_tune_cache;
+struct TunedLaunch {
+  int cfg, x_chunk, axis_split, tb, tb_chunk;
+  bool sweep;
+};
+std::map<std::tuple<int, int, int, int, int>, TunedLaunch> g_tune_cache;
 
 }  // namespace
 
@@ -321,14 +327,22 @@ struct jxf_grid3d {
   int n_tb_shell = 0, n_tb_inner = 0;
   int n_tb_shell_ax[6] = {0, 0, 0, 0, 0, 0};
   int tb_split_cfg = -1, tb_split_chunk = -1, tb_split_axes = -1;
+  // in-place two-pass steps (sweep_registry.h) instead of the TMA launches
+  bool sweep = false;
+  bool sweep_built = false;      // plan and source lists below are current
+  SweepPlan sw{};
+  int* d_sw_ptr = nullptr;       // sources by block (CSR), cells, terms
+  SrcCell* d_sw_cells = nullptr;
+  SrcTerm* d_sw_terms = nullptr;
 };
 
 namespace {
 
 int cells_ok(const jxf_grid3d* g, long long cell) { return cell >= 0 && cell < g->n; }
 
-int build_generic_sources(jxf_grid3d* g) {
-  // group by (cell, comp) in order of first appearance; terms in list order
+// Sources grouped by (cell, comp) in order of first appearance; the terms of
+// a group in list order.
+void group_sources(const jxf_grid3d* g, std::vector<SrcCell>& cells, std::vector<SrcTerm>& terms) {
   std::map<std::pair<long long, int>, std::vector<int>> groups;
   std::vector<std::pair<long long, int>> order;
   for (size_t i = 0; i < g->src_cell.size(); ++i) {
@@ -341,8 +355,6 @@ int build_generic_sources(jxf_grid3d* g) {
       it->second.push_back((int)i);
     }
   }
-  std::vector<SrcCell> cells;
-  std::vector<SrcTerm> terms;
   for (auto& key : order) {
     SrcCell c{};
     c.cell = key.first;
@@ -352,6 +364,12 @@ int build_generic_sources(jxf_grid3d* g) {
     c.count = (int)terms.size() - c.first;
     cells.push_back(c);
   }
+}
+
+int build_generic_sources(jxf_grid3d* g) {
+  std::vector<SrcCell> cells;
+  std::vector<SrcTerm> terms;
+  group_sources(g, cells, terms);
   g->n_cells = (int)cells.size();
   TRY(upload(&g->d_cells, cells, &g->bytes));
   TRY(upload(&g->d_terms, terms, &g->bytes));
@@ -1060,6 +1078,120 @@ int ensure_tb_ready(jxf_grid3d* g) {
   return JXF_OK;
 }
 
+// ---------------------------------------------------------------------------
+// in-place two-pass steps (fdtd3d_sweep.cuh)
+// ---------------------------------------------------------------------------
+
+// Grids the sweep kernels can address: whole grids whose planes and psi arrays
+// have 32-bit offsets and whose planes fit the launch grid's y extent.
+bool sweep_ok(const jxf_grid3d* g) {
+  const long long plane = (long long)g->d.ny * g->d.nz;
+  if (g->slab || plane >= (1LL << 30) || g->d.nx > 65535) return false;
+  if (g->mode != MODE_CPML) return true;
+  return (long long)g->L[0] * plane < (1LL << 31) &&
+         (long long)g->d.nx * g->L[1] * g->d.nz < (1LL << 31) &&
+         (long long)g->d.nx * g->d.ny * g->L[2] < (1LL << 31);
+}
+
+// The work split of a plane (SweepPlan) and the source lists of its blocks.
+int build_sweep(jxf_grid3d* g) {
+  if (g->sweep_built) return JXF_OK;
+  const int nx = g->d.nx, ny = g->d.ny, nz = g->d.nz;
+  const SweepKernels k = sweep_kernels(g->mode, g->kappa, g->cb != nullptr, nz);
+  SweepPlan& s = g->sw;
+  s = SweepPlan{};
+  s.x1 = nx;
+  s.y1 = ny;
+  s.z1 = nz;
+  if (g->mode == MODE_CPML) {
+    s.x0 = g->P[0] < 0 ? 0 : g->P[0];
+    s.x1 = g->P[0] < 0 ? 0 : nx - g->P[0];
+    s.y0 = g->P[1] < 0 ? 0 : g->P[1];
+    s.y1 = g->P[1] < 0 ? 0 : ny - g->P[1];
+    // columns outside the z slabs start and end on 32-byte sectors: the z
+    // regions' loads and stores then share none with them (128^3, 10 layers:
+    // 24.0 us a step against 24.7 on multiples of four cells)
+    const int al = k.v0 > 1 ? 8 : 1;
+    s.z0 = g->P[2] < 0 ? 0 : (g->P[2] + al - 1) / al * al;
+    s.z1 = g->P[2] < 0 ? 0 : (nz - g->P[2]) / al * al;
+    if (s.z1 <= s.z0) s.z0 = s.z1 = 0;
+  }
+  const int slab_rows = s.y0 + ny - s.y1, mid_rows = s.y1 - s.y0;
+  const int slab_w = (s.z0 + nz - s.z1) / k.v1, mid_w = (s.z1 - s.z0) / k.v0;
+  const int rows[4] = {slab_rows, mid_rows, slab_rows, mid_rows};
+  const int w[4] = {slab_w, slab_w, mid_w, mid_w};
+  int base[4];
+  for (int i = 0; i < 4; ++i) {
+    s.r[i].w = w[i];
+    s.r[i].n = rows[i] * w[i];
+    s.r[i].nb = (s.r[i].n + SWEEP_THREADS - 1) / SWEEP_THREADS;
+    s.r[i].dw = make_fastdiv((uint32_t)std::max(w[i], 1));
+    base[i] = s.nblk;
+    s.nblk += s.r[i].nb;
+  }
+  std::vector<SrcCell> cells;
+  std::vector<SrcTerm> terms;
+  group_sources(g, cells, terms);
+  auto block_of = [&](const SrcCell& c) {
+    const int z = (int)(c.cell % nz), y = (int)((c.cell / nz) % ny);
+    const int x = (int)(c.cell / ((long long)nz * ny));
+    const bool ys = y < s.y0 || y >= s.y1, zs = z < s.z0 || z >= s.z1;
+    const int reg = zs ? (ys ? 0 : 1) : (ys ? 2 : 3);
+    const int row = ys ? (y < s.y0 ? y : y - (s.y1 - s.y0)) : y - s.y0;
+    const int col = zs ? (z < s.z0 ? z : z - (s.z1 - s.z0)) : z - s.z0;
+    const int t = row * s.r[reg].w + col / (zs ? k.v1 : k.v0);
+    return (long long)x * s.nblk + base[reg] + t / SWEEP_THREADS;
+  };
+  std::stable_sort(cells.begin(), cells.end(), [&](const SrcCell& u, const SrcCell& v) {
+    return block_of(u) < block_of(v);
+  });
+  std::vector<int> ptr(cells.empty() ? 0 : (size_t)nx * s.nblk + 1, 0);
+  for (const SrcCell& c : cells) ptr[block_of(c) + 1]++;
+  for (size_t i = 1; i < ptr.size(); ++i) ptr[i] += ptr[i - 1];
+  TRY(upload(&g->d_sw_ptr, ptr, &g->bytes));
+  TRY(upload(&g->d_sw_cells, cells, &g->bytes));
+  TRY(upload(&g->d_sw_terms, terms, &g->bytes));
+  s.src_ptr = g->d_sw_ptr;
+  s.src_cell = g->d_sw_cells;
+  s.src_term = g->d_sw_terms;
+  g->sweep_built = true;
+  return JXF_OK;
+}
+
+// One in-place step on buffer set `set` (p.probe_out: row of the state before
+// it, or null; row: row of the state after it, whose H components the E pass
+// records, or null).
+int launch_sweep(jxf_grid3d* g, Step3D& p, int set, float* row, bool sources, cudaStream_t st) {
+  const SweepKernels k = sweep_kernels(g->mode, g->kappa, g->cb != nullptr, g->d.nz);
+  set_io(g, p, set, set);
+  SweepPlan s = g->sw;
+  if (!sources) s.src_ptr = nullptr;
+  float* const before = p.probe_out;
+  for (int half = 0; half < 2; ++half) {
+    p.probe_out = half == 0 ? before : row;
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(s.nblk, g->d.nx, 1);
+    lc.blockDim = dim3(SWEEP_THREADS, 1, 1);
+    lc.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = attr;
+    lc.numAttrs = g->use_pdl ? 1 : 0;
+    cudaError_t e = cudaLaunchKernelEx(&lc, half == 0 ? k.h : k.e, p, s);
+    if (e != cudaSuccess && g->use_pdl) {
+      // stream without programmatic serialization support: launch in order
+      (void)cudaGetLastError();
+      g->use_pdl = false;
+      lc.numAttrs = 0;
+      e = cudaLaunchKernelEx(&lc, half == 0 ? k.h : k.e, p, s);
+    }
+    if (e != cudaSuccess)
+      return fail(JXF_ERR_CUDA, "step kernel launch failed: %s", cudaGetErrorString(e));
+  }
+  return JXF_OK;
+}
+
 int heuristic_tune(jxf_grid3d* g) {
   // Small grids: smaller tiles and chunks keep >= 2 waves of blocks.
   const long long cells = g->n;
@@ -1079,19 +1211,24 @@ int axis_split_override() {
 // and the step counter are untouched, probes off) and keep the fastest.
 int autotune(jxf_grid3d* g, cudaStream_t st) {
   // (x-slabs tune apart from whole grids: they take no blocked passes)
-  const auto key = std::make_tuple(g->d.nx, g->d.ny, g->d.nz,
-                                   g->mode * 4 + (g->kappa ? 1 : 0) + (g->slab ? 2 : 0),
-                                   g->cb ? 1 : 0);
+  // a caller who asked for the TMA path gets TMA launches
+  const bool can_sweep = g->d.path == JXF_PATH_AUTO && sweep_ok(g);
+  const auto key = std::make_tuple(
+      g->d.nx, g->d.ny, g->d.nz,
+      g->mode * 8 + (g->kappa ? 1 : 0) + (g->slab ? 2 : 0) + (can_sweep ? 4 : 0), g->cb ? 1 : 0);
+  g->sweep = false;
   const int split_env = axis_split_override();
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune_cache.find(key);
     if (it != g_tune_cache.end()) {
-      g->cfg = std::get<0>(it->second);
-      g->x_chunk = std::get<1>(it->second);
-      g->axis_split = std::get<2>(it->second);
-      g->tb = std::get<3>(it->second);
-      g->tb_chunk = std::get<4>(it->second);
+      const TunedLaunch& t = it->second;
+      g->cfg = t.cfg;
+      g->x_chunk = t.x_chunk;
+      g->axis_split = t.axis_split;
+      g->tb = t.tb;
+      g->tb_chunk = t.tb_chunk;
+      g->sweep = t.sweep;
       return JXF_OK;
     }
   }
@@ -1129,6 +1266,10 @@ int autotune(jxf_grid3d* g, cudaStream_t st) {
     TRY(heuristic_tune(g));
     g->tb = -1;
     if (split_env >= 0) g->axis_split = split_env;
+    // below 2^18 cells the TMA launches have too few blocks in flight and a
+    // sweep is bound by its two launches (60^3 absorbing: 5.0 us a step
+    // against 11 us)
+    g->sweep = can_sweep && g->n < (1LL << 18);
   } else {
     cudaEvent_t e0, e1;
     CUDA_TRY(cudaEventCreate(&e0));
@@ -1220,6 +1361,26 @@ int autotune(jxf_grid3d* g, cudaStream_t st) {
         }
       }
     }
+    // in-place sweeps, on the idle buffer set
+    if (can_sweep && split_env < 0) {
+      TRY(build_sweep(g));
+      Step3D p = base_params(g);
+      TRY(launch_sweep(g, p, 1 - g->cur, nullptr, false, st));
+      const int reps = g->n >= (1LL << 25) ? 3 : (g->n >= (1LL << 21) ? 40 : 100);
+      for (int trial = 0; trial < 2; ++trial) {
+        CUDA_TRY(cudaEventRecord(e0, st));
+        for (int r = 0; r < reps; ++r)
+          TRY(launch_sweep(g, p, 1 - g->cur, nullptr, false, st));
+        CUDA_TRY(cudaEventRecord(e1, st));
+        CUDA_TRY(cudaEventSynchronize(e1));
+        float t = 0;
+        CUDA_TRY(cudaEventElapsedTime(&t, e0, e1));
+        if (t / (float)reps < best) {
+          best = t / (float)reps;
+          g->sweep = true;
+        }
+      }
+    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     g->cfg = bc;
@@ -1235,12 +1396,14 @@ int autotune(jxf_grid3d* g, cudaStream_t st) {
     // overwrites before anything reads it.
   }
   std::lock_guard<std::mutex> lk(g_tune_mu);
-  g_tune_cache[key] = std::make_tuple(g->cfg, g->x_chunk, g->axis_split, g->tb, g->tb_chunk);
+  g_tune_cache[key] =
+      TunedLaunch{g->cfg, g->x_chunk, g->axis_split, g->tb, g->tb_chunk, g->sweep};
   return JXF_OK;
 }
 
 int ensure_tma_ready(jxf_grid3d* g, cudaStream_t st) {
   if (g->cfg < 0) TRY(autotune(g, st));
+  if (g->sweep) return build_sweep(g);
   if (!g->maps_ok) TRY(encode_maps(g));
   if (!g->src_cell.empty() && (g->built_cfg != g->cfg || g->built_chunk != g->x_chunk))
     TRY(build_tma_sources(g));
@@ -1486,6 +1649,9 @@ int jxf_grid3d_destroy(jxf_grid3d* g) {
   dfree(g->d_tb_shell);
   for (int a = 0; a < 6; ++a) dfree(g->d_tb_shell_ax[a]);
   dfree(g->d_tb_inner);
+  dfree(g->d_sw_ptr);
+  dfree(g->d_sw_cells);
+  dfree(g->d_sw_terms);
   dfree(g->adj_ck);
   dfree(g->adj_sg);
   dfree(g->adj_l);
@@ -1506,7 +1672,8 @@ int jxf_grid3d_get_info(const jxf_grid3d* g, jxf_grid3d_info* out) {
   out->coef_e = g->coef_e;
   out->step = g->step;
   out->path = g->path;
-  if (g->path == JXF_PATH_TMA && g->cfg >= 0) {
+  const bool tma = g->path == JXF_PATH_TMA && !g->sweep;
+  if (tma && g->cfg >= 0) {
     const TmaConfig& c = tma_configs()[g->cfg];
     out->tile_z = c.tz;
     out->tile_y = c.ty;
@@ -1519,11 +1686,11 @@ int jxf_grid3d_get_info(const jxf_grid3d* g, jxf_grid3d_info* out) {
   out->device_bytes = g->bytes;
   out->shell_blocks = g->n_shell + g->n_shell_ax[0] + g->n_shell_ax[1] + g->n_shell_ax[2];
   out->interior_blocks = g->n_inner;
-  out->tma_config = g->path == JXF_PATH_TMA ? g->cfg : -1;
+  out->tma_config = tma ? g->cfg : -1;
   out->axis_split = g->axis_split;
-  out->blocked_config = g->path == JXF_PATH_TMA ? g->tb : -1;
-  out->blocked_x_chunk = g->path == JXF_PATH_TMA && g->tb >= 0 ? g->tb_chunk : 0;
-  if (g->path == JXF_PATH_TMA && g->tb >= 0)
+  out->blocked_config = tma ? g->tb : -1;
+  out->blocked_x_chunk = tma && g->tb >= 0 ? g->tb_chunk : 0;
+  if (tma && g->tb >= 0)
     out->blocked_kernels_per_pass =
         g->mode != MODE_CPML || g->tb_split_cfg < 0
             ? 1
@@ -1533,7 +1700,9 @@ int jxf_grid3d_get_info(const jxf_grid3d* g, jxf_grid3d_info* out) {
                   (g->n_tb_shell_ax[4] > 0 ? 1 : 0) + (g->n_tb_shell_ax[5] > 0 ? 1 : 0);
   else
     out->blocked_kernels_per_pass = 0;
-  if (g->path == JXF_PATH_GENERIC)
+  if (g->sweep || (g->path == JXF_PATH_GENERIC && sweep_ok(g)))
+    out->kernels_per_step = 2;
+  else if (g->path == JXF_PATH_GENERIC)
     out->kernels_per_step = 2 + (g->n_cells > 0 ? 1 : 0);
   else if (g->mode == MODE_CPML && g->split_cfg >= 0)
     out->kernels_per_step = (g->n_shell > 0 ? 1 : 0) + (g->n_inner > 0 ? 1 : 0) +
@@ -1553,6 +1722,7 @@ int jxf_grid3d_set_launch(jxf_grid3d* g, int32_t cfg, int32_t x_chunk) {
   if (cfg >= 0 && x_chunk < 1) return fail(JXF_ERR_INVALID, "x_chunk must be >= 1");
   g->cfg = cfg;
   g->x_chunk = x_chunk;
+  g->sweep = false;
   g->maps_ok = false;
   g->built_cfg = -1;
   return JXF_OK;
@@ -1570,6 +1740,7 @@ int jxf_grid3d_set_blocked(jxf_grid3d* g, int32_t cfg, int32_t x_chunk) {
   if (g->cfg < 0) TRY(heuristic_tune(g));  // one-step shape for odd remainders
   g->tb = cfg < 0 ? -1 : cfg;
   g->tb_chunk = cfg < 0 ? 0 : x_chunk;
+  g->sweep = false;
   g->maps_tb_ok = false;
   g->tb_built_cfg = -1;
   g->tb_split_cfg = -1;
@@ -1643,6 +1814,7 @@ int jxf_grid3d_set_sources(jxf_grid3d* g, int32_t n, const int64_t* cell, const 
   TRY(build_generic_sources(g));
   g->built_cfg = -1;
   g->tb_built_cfg = -1;
+  g->sweep_built = false;
   return JXF_OK;
 }
 
@@ -1711,8 +1883,23 @@ int jxf_grid3d_step(jxf_grid3d* g, int32_t n_steps, float* probe_out, void* stre
   cudaStream_t st = (cudaStream_t)stream;
   Step3D p = base_params(g);
   const int np = g->n_probes;
-  if (g->path == JXF_PATH_TMA) {
-    TRY(ensure_tma_ready(g, st));
+  if (g->path == JXF_PATH_TMA) TRY(ensure_tma_ready(g, st));
+  if (g->sweep || (g->path == JXF_PATH_GENERIC && sweep_ok(g))) {
+    TRY(build_sweep(g));
+    // a learned band corrects the state after the E pass, so its probes are
+    // gathered after it
+    const bool record = probe_out && np > 0;
+    for (int k = 0; k < n_steps; ++k) {
+      float* const row = record ? probe_out + (size_t)k * np : nullptr;
+      const bool fused = record && !g->band.band;
+      p.step = g->step;
+      p.probe_out = fused && k > 0 ? row - np : nullptr;
+      TRY(launch_sweep(g, p, g->cur, fused ? row : nullptr, !g->src_cell.empty(), st));
+      g->step++;
+      if (g->band.band) TRY(band_launch(g->band, st, g->cur));
+      if (record && (g->band.band || k + 1 == n_steps)) TRY(gather_probes(g, g->cur, row, st));
+    }
+  } else if (g->path == JXF_PATH_TMA) {
     p.blk_src_ptr = g->src_cell.empty() ? nullptr : g->d_blk_ptr;
     p.src = g->d_entries;
     for (int k = 0; k < n_steps;) {
