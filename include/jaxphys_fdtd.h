@@ -354,6 +354,12 @@ int jxf_grid2d_set_walls(jxf_grid2d* g, int32_t n, const int32_t* y,
                          const int32_t* gap_start, const int32_t* gap_end);
 /* Replaces the scan over fdtd.py:304-364. */
 int jxf_grid2d_step(jxf_grid2d* g, int32_t n_steps, void* stream);
+/* Advance n_steps and keep the states after steps 1, 1 + save_every,
+ * 1 + 2 save_every, ... (n_frames of them, all within n_steps; the frames the
+ * reference keeps, fdtd.py:371-377): frame k of a component goes to its buffer
+ * (device memory) at offset k nx ny. */
+int jxf_grid2d_run(jxf_grid2d* g, int32_t n_steps, int32_t save_every, int64_t n_frames,
+                   float* ez, float* hx, float* hy, void* stream);
 int jxf_grid2d_reset(jxf_grid2d* g, void* stream);
 int jxf_grid2d_field_ptr(jxf_grid2d* g, int32_t comp, float** out);
 int jxf_grid2d_get_field(jxf_grid2d* g, int32_t comp, float* dst, int32_t dst_is_host,

@@ -154,6 +154,7 @@ SIGNATURES = {
     "jxf_grid2d_set_waveforms": (C.c_int, [_vp, _i32, _i64, _vp]),
     "jxf_grid2d_set_walls": (C.c_int, [_vp, _i32, _vp, _vp, _vp]),
     "jxf_grid2d_step": (C.c_int, [_vp, _i32, _vp]),
+    "jxf_grid2d_run": (C.c_int, [_vp, _i32, _i32, _i64, _vp, _vp, _vp, _vp]),
     "jxf_grid2d_reset": (C.c_int, [_vp, _vp]),
     "jxf_grid2d_field_ptr": (C.c_int, [_vp, _i32, C.POINTER(_vp)]),
     "jxf_grid2d_get_field": (C.c_int, [_vp, _i32, _vp, _i32, _vp]),

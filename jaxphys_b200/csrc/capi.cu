@@ -2243,7 +2243,233 @@ struct jxf_grid2d {
   int* d_wall_g0 = nullptr;
   int* d_wall_g1 = nullptr;
   long long step = 0;
+  // second buffer set of the several-steps launches; between API calls the
+  // state is in f
+  float* f2[3] = {};
+  bool no_f2 = false;   // its allocation failed: one step per launch
+  bool use_pdl = true;  // programmatic dependent launch between step kernels
 };
+
+namespace {
+
+// Launch shapes of k2d_steps: window columns, strips, rows per strip.
+struct Block2DConfig {
+  int w, rows, threads;
+  size_t smem;
+  void (*k[3])(const Block2D);  // absorbing, periodic, mirrored
+  // time model of a launch of k steps in microseconds, absorbing and other
+  // grids: launch + (k + 2) max(latency of a window's step, windows per SM
+  // times their throughput); loading and storing a window costs about two
+  // steps.  Fitted to 64^2 .. 2000 x 1500 grids on one B200 (1024^2 absorbing,
+  // 10 steps: shape 0 98 us, shape 1 34 us; 64^2: 8.2 and 15.3 us).
+  double launch, lat[2], thr[2];
+};
+template <int W, int NS, int R>
+Block2DConfig make_block2d(double launch, double lat0, double lat1, double thr0, double thr1) {
+  return {W,
+          NS * R,
+          B2DLayout<W, NS, R>::NT,
+          B2DLayout<W, NS, R>::SMEM_BYTES,
+          {k2d_steps<MODE_ABSORB, W, NS, R>, k2d_steps<MODE_PERIODIC, W, NS, R>,
+           k2d_steps<MODE_PEC, W, NS, R>},
+          launch,
+          {lat0, lat1},
+          {thr0, thr1}};
+}
+const std::vector<Block2DConfig>& block2d_configs() {
+  static const std::vector<Block2DConfig> c = {
+      make_block2d<32, 16, 2>(3.4, 0.48, 0.70, 0.21, 0.23),
+      make_block2d<64, 16, 4>(5.6, 0.82, 1.28, 0.62, 0.72)};
+  return c;
+}
+
+int block2d_halo(const jxf_grid2d* g, int steps) {
+  // the copies between edge cells two apart cost two more cells, once
+  return g->mode == MODE_ABSORB ? steps : steps + 2;
+}
+
+bool block2d_fits(const jxf_grid2d* g, const Block2DConfig& c, int steps) {
+  const int h = block2d_halo(g, steps);
+  if (steps < 1 || steps > B2D_MAX_STEPS || c.w - 2 * h < 4 || c.rows - 2 * h < 4) return false;
+  // a validity front crosses one pair of wrapped edges at most
+  if (g->mode == MODE_PERIODIC && std::min(g->d.nx, g->d.ny) < steps + 4) return false;
+  const int th = c.rows - 2 * h;
+  return (g->d.nx + th - 1) / th <= 65535;
+}
+
+// Launch shape for runs of n steps: the (shape, steps per launch) of least
+// modelled time.  JXF_BLOCK2D="shape,steps" pins it where it fits.
+bool block2d_choose(const jxf_grid2d* g, int n, int* cfg, int* steps) {
+  const auto& cs = block2d_configs();
+  if (const char* e = std::getenv("JXF_BLOCK2D")) {
+    int c = -1, k = -1;
+    if (std::sscanf(e, "%d,%d", &c, &k) == 2 && c >= 0 && c < (int)cs.size() &&
+        block2d_fits(g, cs[c], std::min(k, n))) {
+      *cfg = c;
+      *steps = std::min(k, n);
+      return true;
+    }
+  }
+  double best = 1e30;
+  for (int c = 0; c < (int)cs.size(); ++c)
+    for (int k = 1; k <= std::min(n, B2D_MAX_STEPS); ++k) {
+      if (!block2d_fits(g, cs[c], k)) continue;
+      const int h = block2d_halo(g, k);
+      const long long th = cs[c].rows - 2 * h, tw = cs[c].w - 2 * h;
+      const long long tiles = ((g->d.nx + th - 1) / th) * ((g->d.ny + tw - 1) / tw);
+      const int post = g->mode == MODE_ABSORB ? 0 : 1;
+      const int m = (n + k - 1) / k;  // launches, of n / m steps
+      const double step =
+          std::max(cs[c].lat[post], (double)((tiles + 147) / 148) * cs[c].thr[post]);
+      const double t = m * cs[c].launch + (n + 2 * m) * step;
+      if (t < best) {
+        best = t;
+        *cfg = c;
+        *steps = k;
+      }
+    }
+  return best < 1e30;
+}
+
+bool block2d_ready(jxf_grid2d* g) {
+  if (g->no_f2) return false;
+  if (g->f2[0]) return true;
+  for (int k = 0; k < 3; ++k)
+    if (dmalloc(&g->f2[k], (size_t)g->n, &g->bytes) != JXF_OK) {
+      (void)cudaGetLastError();
+      for (int i = 0; i < k; ++i) {
+        g->bytes -= g->n * 4;
+        dfree(g->f2[i]);
+      }
+      g->no_f2 = true;
+      return false;
+    }
+  return true;
+}
+
+// n steps in launches of `steps` or fewer (of nearly equal length; an even
+// number of launches if even), from set *set on; the state after the last
+// goes to `frame` too (null: no frame).
+int block2d_advance(jxf_grid2d* g, Step2D& p, int cfg, int steps, int n, bool even,
+                    float* const* frame, int* set, cudaStream_t st) {
+  const Block2DConfig& c = block2d_configs()[cfg];
+  auto* const kern = c.k[g->mode == MODE_ABSORB ? 0 : (g->mode == MODE_PERIODIC ? 1 : 2)];
+  if (c.smem > 48 * 1024) {
+    static std::mutex mu;
+    static std::map<std::pair<void (*)(const Block2D), int>, bool> done;
+    std::lock_guard<std::mutex> lk(mu);
+    bool& have = done[{kern, g->d.device}];
+    if (!have)
+      CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem));
+    have = true;
+  }
+  int m = (n + steps - 1) / steps;
+  if (even && m % 2 == 1 && m < n) ++m;
+  Block2D b{};
+  for (int i = 0; i < m; ++i) {
+    const int k = n / m + (i < n % m ? 1 : 0);
+    b.p = p;
+    b.p.step = g->step;
+    b.steps = k;
+    b.halo = block2d_halo(g, k);
+    for (int f = 0; f < 3; ++f) {
+      b.in[f] = *set ? g->f2[f] : g->f[f];
+      b.out[f] = *set ? g->f[f] : g->f2[f];
+      b.frame[f] = frame && i + 1 == m ? frame[f] : nullptr;
+    }
+    const int th = c.rows - 2 * b.halo, tw = c.w - 2 * b.halo;
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3((g->d.ny + tw - 1) / tw, (g->d.nx + th - 1) / th, 1);
+    lc.blockDim = dim3(c.threads, 1, 1);
+    lc.dynamicSmemBytes = c.smem;
+    lc.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = attr;
+    lc.numAttrs = g->use_pdl ? 1 : 0;
+    cudaError_t e = cudaLaunchKernelEx(&lc, kern, b);
+    if (e != cudaSuccess && g->use_pdl) {
+      // stream without programmatic serialization support: launch in order
+      (void)cudaGetLastError();
+      g->use_pdl = false;
+      lc.numAttrs = 0;
+      e = cudaLaunchKernelEx(&lc, kern, b);
+    }
+    if (e != cudaSuccess)
+      return fail(JXF_ERR_CUDA, "2D step launch failed: %s", cudaGetErrorString(e));
+    g->step += k;
+    *set ^= 1;
+  }
+  return JXF_OK;
+}
+
+// Leaves the state of set `set` in f.
+int block2d_settle(jxf_grid2d* g, int set, cudaStream_t st) {
+  for (int f = 0; f < 3 && set; ++f)
+    CUDA_TRY(cudaMemcpyAsync(g->f[f], g->f2[f], (size_t)g->n * 4, cudaMemcpyDeviceToDevice, st));
+  return JXF_OK;
+}
+
+int check_waves2d(const jxf_grid2d* g, long long n_steps) {
+  if (g->n_src == 0) return JXF_OK;
+  int max_w = 0;
+  for (int w : g->src_wave) max_w = std::max(max_w, w);
+  if (max_w >= g->n_waves)
+    return fail(JXF_ERR_INVALID, "source wave id %d has no waveform row", max_w);
+  if (g->step + n_steps > g->wave_len)
+    return fail(JXF_ERR_INVALID, "waveform table covers %lld steps, need %lld", g->wave_len,
+                g->step + n_steps);
+  return JXF_OK;
+}
+
+Step2D step2d_params(jxf_grid2d* g) {
+  Step2D p{};
+  p.nx = g->d.nx;
+  p.ny = g->d.ny;
+  p.a = (float)g->coef_h;
+  p.b = (float)g->coef_e;
+  p.ez = g->f[0];
+  p.hx = g->f[1];
+  p.hy = g->f[2];
+  p.damp[0] = g->damp[0];
+  p.damp[1] = g->damp[1];
+  p.n_src = g->n_src;
+  p.src_y = g->d_src_y;
+  p.src_amp = g->d_src_amp;
+  p.src_wave = g->d_src_wave;
+  p.wave = g->d_wave;
+  p.wave_len = g->wave_len;
+  p.n_wall = g->n_wall;
+  p.wall_y = g->d_wall_y;
+  p.wall_g0 = g->d_wall_g0;
+  p.wall_g1 = g->d_wall_g1;
+  return p;
+}
+
+// One step per launch sequence, in place.
+int step2d_single(jxf_grid2d* g, Step2D& p, cudaStream_t st) {
+  const int threads = 256;
+  const int blocks = (int)std::min<long long>((g->n + threads - 1) / threads, 148LL * 16);
+  p.step = g->step;
+  if (g->mode == MODE_PERIODIC) {
+    k2d_h<MODE_PERIODIC><<<blocks, threads, 0, st>>>(p);
+    k2d_e<MODE_PERIODIC, false><<<blocks, threads, 0, st>>>(p);
+    k2d_post<MODE_PERIODIC><<<1, 1024, 0, st>>>(p);
+  } else if (g->mode == JXF_BND_REFLECTING) {
+    k2d_h<MODE_ABSORB><<<blocks, threads, 0, st>>>(p);
+    k2d_e<MODE_PEC, false><<<blocks, threads, 0, st>>>(p);
+    k2d_post<MODE_ABSORB><<<1, 1024, 0, st>>>(p);
+  } else {
+    k2d_h<MODE_ABSORB><<<blocks, threads, 0, st>>>(p);
+    k2d_e<MODE_ABSORB, true><<<blocks, threads, 0, st>>>(p);
+  }
+  CUDA_TRY(cudaGetLastError());
+  g->step++;
+  return JXF_OK;
+}
+
+}  // namespace
 
 extern "C" {
 
@@ -2299,6 +2525,7 @@ int jxf_grid2d_destroy(jxf_grid2d* g) {
   if (!g) return JXF_OK;
   DeviceGuard dg(g->d.device);
   for (int k = 0; k < 3; ++k) dfree(g->f[k]);
+  for (int k = 0; k < 3; ++k) dfree(g->f2[k]);
   for (int k = 0; k < 2; ++k) dfree(g->damp[k]);
   dfree(g->d_src_y);
   dfree(g->d_src_amp);
@@ -2363,57 +2590,55 @@ int jxf_grid2d_step(jxf_grid2d* g, int32_t n_steps, void* stream) {
   if (!g) return fail(JXF_ERR_INVALID, "null handle");
   if (n_steps < 0) return fail(JXF_ERR_INVALID, "n_steps must be >= 0");
   if (n_steps == 0) return JXF_OK;
-  if (g->n_src > 0) {
-    int max_w = 0;
-    for (int w : g->src_wave) max_w = std::max(max_w, w);
-    if (max_w >= g->n_waves)
-      return fail(JXF_ERR_INVALID, "source wave id %d has no waveform row", max_w);
-    if (g->step + n_steps > g->wave_len)
-      return fail(JXF_ERR_INVALID, "waveform table covers %lld steps, need %lld", g->wave_len,
-                  g->step + n_steps);
-  }
+  TRY(check_waves2d(g, n_steps));
   DeviceGuard dg(g->d.device);
   cudaStream_t st = (cudaStream_t)stream;
-  Step2D p{};
-  p.nx = g->d.nx;
-  p.ny = g->d.ny;
-  p.a = (float)g->coef_h;
-  p.b = (float)g->coef_e;
-  p.ez = g->f[0];
-  p.hx = g->f[1];
-  p.hy = g->f[2];
-  p.damp[0] = g->damp[0];
-  p.damp[1] = g->damp[1];
-  p.n_src = g->n_src;
-  p.src_y = g->d_src_y;
-  p.src_amp = g->d_src_amp;
-  p.src_wave = g->d_src_wave;
-  p.wave = g->d_wave;
-  p.wave_len = g->wave_len;
-  p.n_wall = g->n_wall;
-  p.wall_y = g->d_wall_y;
-  p.wall_g0 = g->d_wall_g0;
-  p.wall_g1 = g->d_wall_g1;
-  const int threads = 256;
-  const int blocks = (int)std::min<long long>((g->n + threads - 1) / threads, 148LL * 16);
-  for (int k = 0; k < n_steps; ++k) {
-    p.step = g->step;
-    if (g->mode == MODE_PERIODIC) {
-      k2d_h<MODE_PERIODIC><<<blocks, threads, 0, st>>>(p);
-      k2d_e<MODE_PERIODIC, false><<<blocks, threads, 0, st>>>(p);
-      k2d_post<MODE_PERIODIC><<<1, 1024, 0, st>>>(p);
-    } else if (g->mode == JXF_BND_REFLECTING) {
-      k2d_h<MODE_ABSORB><<<blocks, threads, 0, st>>>(p);
-      k2d_e<MODE_PEC, false><<<blocks, threads, 0, st>>>(p);
-      k2d_post<MODE_ABSORB><<<1, 1024, 0, st>>>(p);
-    } else {
-      k2d_h<MODE_ABSORB><<<blocks, threads, 0, st>>>(p);
-      k2d_e<MODE_ABSORB, true><<<blocks, threads, 0, st>>>(p);
-    }
-    CUDA_TRY(cudaGetLastError());
-    g->step++;
+  Step2D p = step2d_params(g);
+  // one step: in place (a launch of several would have to copy back)
+  int cfg = 0, steps = 0, set = 0;
+  if (n_steps >= 2 && block2d_choose(g, n_steps, &cfg, &steps) && block2d_ready(g)) {
+    TRY(block2d_advance(g, p, cfg, steps, n_steps, true, nullptr, &set, st));
+    return block2d_settle(g, set, st);
   }
+  for (int k = 0; k < n_steps; ++k) TRY(step2d_single(g, p, st));
   return JXF_OK;
+}
+
+int jxf_grid2d_run(jxf_grid2d* g, int32_t n_steps, int32_t save_every, int64_t n_frames, float* ez,
+                   float* hx, float* hy, void* stream) {
+  if (!g) return fail(JXF_ERR_INVALID, "null handle");
+  if (n_steps < 0 || save_every < 1 || n_frames < 0)
+    return fail(JXF_ERR_INVALID, "n_steps and n_frames must be >= 0, save_every >= 1");
+  if (n_frames > 0 && (!ez || !hx || !hy)) return fail(JXF_ERR_INVALID, "null frame buffer");
+  if (n_frames > 0 && 1 + (n_frames - 1) * (int64_t)save_every > n_steps)
+    return fail(JXF_ERR_INVALID, "%lld frames do not fit in %d steps", (long long)n_frames, n_steps);
+  if (n_steps == 0) return JXF_OK;
+  TRY(check_waves2d(g, n_steps));
+  DeviceGuard dg(g->d.device);
+  cudaStream_t st = (cudaStream_t)stream;
+  Step2D p = step2d_params(g);
+  float* const frames[3] = {ez, hx, hy};
+  const long long first = g->step;
+  int set = 0;
+  // the launch shape follows from the usual run between two frames
+  int cfg = 0, steps = 0;
+  const int usual = n_frames > 1 ? save_every : n_steps;
+  const bool blocked = block2d_choose(g, usual, &cfg, &steps) && block2d_ready(g);
+  for (int64_t k = 0; k <= n_frames; ++k) {
+    const bool save = k < n_frames;
+    const int n = (int)(first + (save ? 1 + k * (int64_t)save_every : n_steps) - g->step);
+    float* at[3];
+    for (int f = 0; f < 3; ++f) at[f] = save ? frames[f] + k * g->n : nullptr;
+    if (n == 0) continue;
+    if (blocked) {
+      TRY(block2d_advance(g, p, cfg, steps, n, false, save ? at : nullptr, &set, st));
+      continue;
+    }
+    for (int i = 0; i < n; ++i) TRY(step2d_single(g, p, st));
+    for (int f = 0; f < 3 && save; ++f)
+      CUDA_TRY(cudaMemcpyAsync(at[f], g->f[f], (size_t)g->n * 4, cudaMemcpyDeviceToDevice, st));
+  }
+  return block2d_settle(g, set, st);
 }
 
 int jxf_grid2d_reset(jxf_grid2d* g, void* stream) {

@@ -53,11 +53,6 @@ __device__ __forceinline__ long long zs_index(int x, int y, int km, int ny, int 
   return ((long long)x * ny + y) * L2 + km;
 }
 
-template <bool B>
-struct BoolC {
-  static constexpr bool value = B;
-};
-
 // One CPML term of a field component: the derivative along one axis.
 struct PsiTerm {
   bool on;     // cell inside this axis' slab (psi stored)

@@ -90,6 +90,12 @@ __device__ __forceinline__ void decode_cell(long long idx, int nz, int ny, bool 
   }
 }
 
+// a compile-time bool as a function argument
+template <bool B>
+struct BoolC {
+  static constexpr bool value = B;
+};
+
 struct CpmlDev {
   const float* tab[3][TAB_COUNT];  // per axis, length n_axis
   int L[3];                        // slab storage extent per axis

@@ -221,16 +221,10 @@ class EMGrid:
                 for _ in range(3)]
         lib = nat.load()
         st = nat.stream_handle()
-        done = 0
-        for s, k in enumerate(saved):
-            if k + 1 > done:
-                nat.check(lib.jxf_grid2d_step(self._h, k + 1 - done, st), "jxf_grid2d_step")
-                done = k + 1
-            for c in range(3):
-                nat.check(lib.jxf_grid2d_get_field(self._h, c, hist[c][s].data_ptr(), 0, st),
-                          "get_field")
-        if n_steps > done:
-            nat.check(lib.jxf_grid2d_step(self._h, n_steps - done, st), "jxf_grid2d_step")
+        if n_steps > 0:
+            nat.check(lib.jxf_grid2d_run(self._h, n_steps, stride, len(saved), hist[0].data_ptr(),
+                                         hist[1].data_ptr(), hist[2].data_ptr(), st),
+                      "jxf_grid2d_run")
         nat.check(lib.jxf_grid2d_check_error(self._h, st), "device error")
         t = np.array([t_start + k * dt + dt for k in saved], dtype=np.float64)
         gx = np.arange(nx) * dx
