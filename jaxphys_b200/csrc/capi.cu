@@ -1124,7 +1124,7 @@ int build_sweep(jxf_grid3d* g) {
   for (int i = 0; i < 4; ++i) {
     s.r[i].w = w[i];
     s.r[i].n = rows[i] * w[i];
-    s.r[i].nb = (s.r[i].n + SWEEP_THREADS - 1) / SWEEP_THREADS;
+    s.r[i].nb = (s.r[i].n + k.threads - 1) / k.threads;
     s.r[i].dw = make_fastdiv((uint32_t)std::max(w[i], 1));
     base[i] = s.nblk;
     s.nblk += s.r[i].nb;
@@ -1140,7 +1140,7 @@ int build_sweep(jxf_grid3d* g) {
     const int row = ys ? (y < s.y0 ? y : y - (s.y1 - s.y0)) : y - s.y0;
     const int col = zs ? (z < s.z0 ? z : z - (s.z1 - s.z0)) : z - s.z0;
     const int t = row * s.r[reg].w + col / (zs ? k.v1 : k.v0);
-    return (long long)x * s.nblk + base[reg] + t / SWEEP_THREADS;
+    return (long long)x * s.nblk + base[reg] + t / k.threads;
   };
   std::stable_sort(cells.begin(), cells.end(), [&](const SrcCell& u, const SrcCell& v) {
     return block_of(u) < block_of(v);
@@ -1171,7 +1171,7 @@ int launch_sweep(jxf_grid3d* g, Step3D& p, int set, float* row, bool sources, cu
     p.probe_out = half == 0 ? before : row;
     cudaLaunchConfig_t lc{};
     lc.gridDim = dim3(s.nblk, g->d.nx, 1);
-    lc.blockDim = dim3(SWEEP_THREADS, 1, 1);
+    lc.blockDim = dim3(k.threads, 1, 1);
     lc.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

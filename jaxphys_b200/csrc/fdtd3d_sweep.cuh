@@ -27,11 +27,25 @@
 
 namespace jxf {
 
-constexpr int SWEEP_THREADS = 128;
+// Threads per block.  128: a block of a CPML region holds few rows, and more
+// threads leave more of them idle.  With one or two cells per thread and no
+// slabs a block of 128 is done so soon that dispatching blocks bounds the pass
+// (128^3 of one cell per thread, absorbing: 35.6 us a step against 22.4 with
+// 256 threads).
+__host__ __device__ constexpr int sweep_threads(int mode, int v0) {
+  return mode != MODE_CPML && v0 < 4 ? 256 : 128;
+}
+// Blocks per SM the compiler must leave registers for: 64 a thread (CPML: 128).
+// Without the bound it keeps fewer loads in flight to fit more blocks, 17.1
+// against 14.3 us a step for the absorbing 128^3 grid; a tighter bound spills
+// the CPML kernel.
+__host__ __device__ constexpr int sweep_min_blocks(int mode, int v0) {
+  return (mode == MODE_CPML ? 512 : 1024) / sweep_threads(mode, v0);
+}
 
 // Work split of one plane x.  CPML grids: the cells of a plane fall in four
 // regions by whether their y / z lies in a psi slab, each cut into blocks of
-// SWEEP_THREADS threads (V0 cells per thread outside the z slabs, V1 inside),
+// sweep_threads() threads (V0 cells per thread outside the z slabs, V1 inside),
 // so that a block runs code for its slabs alone: with one code for all, every
 // warp of a 128-cell row holds z-slab lanes and pays for the CPML update (37
 // against 25 us a step at 128^3).  Other grids: one region.
@@ -284,8 +298,8 @@ __device__ __forceinline__ void sweep_cells(const Step3D& p, int x, int y, int z
 template <bool H, int MODE, int V0, int V1, bool KAPPA, bool CBARR, int REG>
 __device__ __forceinline__ void sweep_region(const Step3D& p, const SweepPlan& s, int x, int b) {
   constexpr bool YS = REG == 0 || REG == 2, ZS = REG < 2;
-  constexpr int V = ZS ? V1 : V0;
-  const int t = b * SWEEP_THREADS + (int)threadIdx.x;
+  constexpr int V = ZS ? V1 : V0, NT = sweep_threads(MODE, V0);
+  const int t = b * NT + (int)threadIdx.x;
   if (t >= s.r[REG].n) return;
   const int j = (int)fdiv((uint32_t)t, s.r[REG].dw);
   const int k = (t - j * s.r[REG].w) * V;
@@ -298,10 +312,11 @@ __device__ __forceinline__ void sweep_region(const Step3D& p, const SweepPlan& s
 // Block b of plane x of one grid.
 template <bool H, int MODE, int V0, int V1, bool KAPPA, bool CBARR>
 __device__ __forceinline__ void sweep_block(const Step3D& p, const SweepPlan& s, int x, int b) {
+  constexpr int NT = sweep_threads(MODE, V0);
   // probes of the state after the previous step: its E components are final
   // until this step's E pass, its H components were recorded by its E pass
   if (p.probe_out != nullptr && b == 0 && x == 0) {
-    for (int i = threadIdx.x; i < p.n_probes; i += SWEEP_THREADS) {
+    for (int i = threadIdx.x; i < p.n_probes; i += NT) {
       const int c = p.probe_comp[i];
       if ((c < 3) == H) p.probe_out[i] = p.in[c][p.probe_cell[i]];
     }
@@ -313,7 +328,7 @@ __device__ __forceinline__ void sweep_block(const Step3D& p, const SweepPlan& s,
     s1 = __ldg(q + 1);
   }
   if (MODE != MODE_CPML) {
-    const int t = b * SWEEP_THREADS + (int)threadIdx.x;
+    const int t = b * NT + (int)threadIdx.x;
     if (t < s.r[3].n) {
       const int y = (int)fdiv((uint32_t)t, s.r[3].dw);
       sweep_cells<H, MODE, V0, KAPPA, CBARR, false, false, false>(p, x, y, (t - y * s.r[3].w) * V0);
@@ -330,7 +345,7 @@ __device__ __forceinline__ void sweep_block(const Step3D& p, const SweepPlan& s,
   // soft sources of the block's cells, after its E update
   if (!H && s0 < s1) {
     __syncthreads();
-    for (int i = s0 + (int)threadIdx.x; i < s1; i += SWEEP_THREADS) {
+    for (int i = s0 + (int)threadIdx.x; i < s1; i += NT) {
       const SrcCell c = s.src_cell[i];
       float* f = p.out[c.comp] + c.cell;
       float v = *f;
@@ -343,11 +358,8 @@ __device__ __forceinline__ void sweep_block(const Step3D& p, const SweepPlan& s,
   }
 }
 
-// (The occupancy bounds leave the compiler 64 and 128 registers: without them
-// it keeps fewer loads in flight to fit more blocks, 17.1 against 14.3 us a
-// step for the absorbing 128^3 grid; a tighter bound spills the CPML kernel.)
 template <bool H, int MODE, int V0, int V1, bool KAPPA, bool CBARR>
-__global__ void __launch_bounds__(SWEEP_THREADS, MODE == MODE_CPML ? 4 : 8)
+__global__ void __launch_bounds__(sweep_threads(MODE, V0), sweep_min_blocks(MODE, V0))
     k3d_sweep(const __grid_constant__ Step3D p, const __grid_constant__ SweepPlan s) {
   grid_dep_wait();
   grid_dep_launch_dependents();

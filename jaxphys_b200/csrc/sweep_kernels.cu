@@ -10,7 +10,7 @@ SweepKernels make(bool cbarr) {
   return SweepKernels{k3d_sweep<true, MODE, V0, V1, KAPPA, false>,
                       cbarr ? k3d_sweep<false, MODE, V0, V1, KAPPA, true>
                             : k3d_sweep<false, MODE, V0, V1, KAPPA, false>,
-                      V0, V1};
+                      V0, V1, sweep_threads(MODE, V0)};
 }
 
 // The widest loads that nz allows (rows of a multiple of V cells keep every

@@ -11,7 +11,8 @@ using SweepKernel = void (*)(const Step3D, const SweepPlan);
 
 struct SweepKernels {
   SweepKernel h, e;
-  int v0, v1;  // cells per thread outside / inside the z slabs
+  int v0, v1;   // cells per thread outside / inside the z slabs
+  int threads;  // per block
 };
 
 // Kernels of a grid: MODE_ABSORB (also PEC with unit tables), MODE_PERIODIC or
