@@ -122,6 +122,12 @@ int jxf_grid3d_set_blocked(jxf_grid3d* g, int32_t cfg, int32_t x_chunk);
  * factor is 0, so Ex, Ey and Ez of that cell keep their initial value (zero);
  * zero, negative and NaN values are rejected. */
 int jxf_grid3d_set_eps_host(jxf_grid3d* g, const double* eps_r);
+
+/* The same from masks (DielectricRegion, fdtd3d.py:58-68,132-137): vacuum, then
+ * eps_r[i] wherever masks[i] is non-zero, in order.  masks: n arrays of
+ * nx*ny*nz bytes in HOST memory; eps_r > 0 or +inf. */
+int jxf_grid3d_set_materials(jxf_grid3d* g, int32_t n, const uint8_t* const* masks,
+                             const double* eps_r);
 /* Same from a DEVICE float32 array (e.g. a DLPack capsule's data pointer):
  * the division runs on the device in FP32 (+inf gives 0, as above). */
 int jxf_grid3d_set_eps_device(jxf_grid3d* g, const float* eps_r, void* stream);
@@ -150,6 +156,13 @@ int jxf_grid3d_set_probes(jxf_grid3d* g, int32_t n, const int64_t* cell,
  * only when the call synchronises; see jxf_grid3d_check_error).  An x-slab
  * (jxf_grid3d_create_slab) takes it only on the TMA path, one step per call. */
 int jxf_grid3d_step(jxf_grid3d* g, int32_t n_steps, float* probe_out, void* stream);
+
+/* Advance n_steps and keep the states after steps 1, 1 + save_every,
+ * 1 + 2 save_every, ... (n_frames of them, all within n_steps; the frames the
+ * reference keeps, fdtd3d.py:396-404): frame k of component c goes to
+ * frames[c] (device memory) at offset k nx ny nz. */
+int jxf_grid3d_run(jxf_grid3d* g, int32_t n_steps, int32_t save_every, int64_t n_frames,
+                   float* const* frames, void* stream);
 
 /* Adjoint (extension; the reference differentiates nothing in its FDTD,
  * and jax.grad through EMGrid3D.simulate, fdtd3d.py:393, would keep every

@@ -106,11 +106,13 @@ SIGNATURES = {
     "jxf_batch3d_launch": (C.c_int, [_vp, C.POINTER(C.c_int32)]),
     "jxf_grid3d_set_blocked": (C.c_int, [_vp, _i32, _i32]),
     "jxf_grid3d_set_eps_host": (C.c_int, [_vp, _vp]),
+    "jxf_grid3d_set_materials": (C.c_int, [_vp, _i32, C.POINTER(_vp), _vp]),
     "jxf_grid3d_set_eps_device": (C.c_int, [_vp, _vp, _vp]),
     "jxf_grid3d_set_sources": (C.c_int, [_vp, _i32, _vp, _vp, _vp, _vp]),
     "jxf_grid3d_set_waveforms": (C.c_int, [_vp, _i32, _i64, _vp]),
     "jxf_grid3d_set_probes": (C.c_int, [_vp, _i32, _vp, _vp]),
     "jxf_grid3d_step": (C.c_int, [_vp, _i32, _vp, _vp]),
+    "jxf_grid3d_run": (C.c_int, [_vp, _i32, _i32, _i64, C.POINTER(_vp), _vp]),
     "jxf_grid3d_reset": (C.c_int, [_vp, _vp]),
     "jxf_grid3d_field_ptr": (C.c_int, [_vp, _i32, C.POINTER(_vp)]),
     "jxf_grid3d_get_field": (C.c_int, [_vp, _i32, _vp, _i32, _vp]),

@@ -283,6 +283,7 @@ struct jxf_grid3d {
   int n_probes = 0;
   int* d_err = nullptr;
   int* d_count = nullptr;
+  uint8_t* d_mask = nullptr;  // staging of a material mask
   // CPML region split: blocks that touch a psi slab (shell) run the CPML
   // kernel, the others the plain kernel (compact block lists per launch shape)
   int* d_shell = nullptr;     // shell blocks touching slabs of several axes
@@ -1661,6 +1662,7 @@ int jxf_grid3d_destroy(jxf_grid3d* g) {
   dfree(g->d_probe_comp);
   dfree(g->d_err);
   dfree(g->d_count);
+  dfree(g->d_mask);
   delete g;
   return JXF_OK;
 }
@@ -1780,6 +1782,65 @@ int jxf_grid3d_set_eps_host(jxf_grid3d* g, const double* eps_r) {
   TRY(upload(&g->cb, cb, &g->bytes));
   g->maps_ok = false;
   g->maps_tb_ok = false;
+  return JXF_OK;
+}
+
+// cb = `in` where the mask is set; elsewhere `out` (fill) or unchanged.
+static __global__ void k_cb_from_mask(const uint8_t* mask, float* cb, float in, float out,
+                                      int fill, long long n) {
+  for (long long i = 4 * ((long long)blockIdx.x * blockDim.x + threadIdx.x); i < n;
+       i += 4 * (long long)gridDim.x * blockDim.x) {
+    if (i + 4 <= n) {
+      const uchar4 m = *reinterpret_cast<const uchar4*>(mask + i);
+      float4 v = make_float4(out, out, out, out);
+      if (!fill) v = *reinterpret_cast<const float4*>(cb + i);
+      if (m.x) v.x = in;
+      if (m.y) v.y = in;
+      if (m.z) v.z = in;
+      if (m.w) v.w = in;
+      *reinterpret_cast<float4*>(cb + i) = v;
+    } else {
+      for (long long k = i; k < n; ++k)
+        if (mask[k] || fill) cb[k] = mask[k] ? in : out;
+    }
+  }
+}
+
+int jxf_grid3d_set_materials(jxf_grid3d* g, int32_t n, const uint8_t* const* masks,
+                             const double* eps_r) {
+  if (!g) return fail(JXF_ERR_INVALID, "null handle");
+  if (n < 0 || (n > 0 && (!masks || !eps_r))) return fail(JXF_ERR_INVALID, "bad material arrays");
+  for (int i = 0; i < n; ++i) {
+    if (!masks[i]) return fail(JXF_ERR_INVALID, "material %d: null mask", i);
+    if (!(eps_r[i] > 0) || std::isnan(eps_r[i]))
+      return fail(JXF_ERR_INVALID, "material %d: eps_r must be positive (or +inf)", i);
+  }
+  if (n == 0) return jxf_grid3d_set_eps_host(g, nullptr);
+  DeviceGuard dg(g->d.device);
+  // steps in flight on any stream may still read the factors
+  CUDA_TRY(cudaDeviceSynchronize());
+  if (!g->cb) TRY(dmalloc(&g->cb, (size_t)g->n, &g->bytes));
+  g->maps_ok = false;
+  g->maps_tb_ok = false;
+  if (!g->d_mask && dmalloc(&g->d_mask, (size_t)g->n, &g->bytes) != JXF_OK) {
+    // no room for the masks: the factors are formed here
+    (void)cudaGetLastError();
+    std::vector<float> cb((size_t)g->n, (float)g->coef_e);
+    for (int i = 0; i < n; ++i)
+      for (long long c = 0; c < g->n; ++c)
+        if (masks[i][c]) cb[c] = (float)(g->coef_e / eps_r[i]);
+    CUDA_TRY(cudaMemcpy(g->cb, cb.data(), cb.size() * 4, cudaMemcpyHostToDevice));
+    return JXF_OK;
+  }
+  const int blocks = (int)std::min<long long>((g->n + 1023) / 1024, 148LL * 8);
+  for (int i = 0; i < n; ++i) {
+    CUDA_TRY(cudaMemcpy(g->d_mask, masks[i], (size_t)g->n, cudaMemcpyHostToDevice));
+    // (one FP64 division and rounding per material, as per cell: fdtd3d.py:299)
+    k_cb_from_mask<<<blocks, 256>>>(g->d_mask, g->cb, (float)(g->coef_e / eps_r[i]),
+                                    (float)g->coef_e, i == 0 ? 1 : 0, g->n);
+    CUDA_TRY(cudaGetLastError());
+  }
+  CUDA_TRY(cudaStreamSynchronize(nullptr));
   return JXF_OK;
 }
 
@@ -2173,6 +2234,55 @@ int jxf_grid3d_snapshot(jxf_grid3d* g, float* dst, void* stream) {
   return JXF_OK;
 }
 
+struct Frame6 {
+  const float* src[6];
+  float* dst[6];
+};
+// The six fields to one frame each (blockIdx.y: component).
+static __global__ void k_frame(const __grid_constant__ Frame6 f, long long n, int vec) {
+  const float* s = f.src[blockIdx.y];
+  float* d = f.dst[blockIdx.y];
+  const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long step = (long long)gridDim.x * blockDim.x;
+  if (vec) {
+    for (long long i = i0; i < n / 4; i += step)
+      reinterpret_cast<float4*>(d)[i] = reinterpret_cast<const float4*>(s)[i];
+  } else {
+    for (long long i = i0; i < n; i += step) d[i] = s[i];
+  }
+}
+
+int jxf_grid3d_run(jxf_grid3d* g, int32_t n_steps, int32_t save_every, int64_t n_frames,
+                   float* const* frames, void* stream) {
+  if (!g) return fail(JXF_ERR_INVALID, "null handle");
+  if (n_steps < 0 || save_every < 1 || n_frames < 0)
+    return fail(JXF_ERR_INVALID, "n_steps and n_frames must be >= 0, save_every >= 1");
+  if (n_frames > 0 && 1 + (n_frames - 1) * (int64_t)save_every > n_steps)
+    return fail(JXF_ERR_INVALID, "%lld frames do not fit in %d steps", (long long)n_frames, n_steps);
+  for (int c = 0; c < 6 && n_frames > 0; ++c)
+    if (!frames || !frames[c]) return fail(JXF_ERR_INVALID, "null frame buffer");
+  DeviceGuard dg(g->d.device);
+  cudaStream_t st = (cudaStream_t)stream;
+  int done = 0;
+  for (int64_t k = 0; k < n_frames; ++k) {
+    const int upto = (int)(1 + k * (int64_t)save_every);
+    TRY(jxf_grid3d_step(g, upto - done, nullptr, stream));
+    done = upto;
+    Frame6 f;
+    bool vec = g->n % 4 == 0;
+    for (int c = 0; c < 6; ++c) {
+      f.src[c] = g->f[g->cur][c];
+      f.dst[c] = frames[c] + k * g->n;
+      vec = vec && reinterpret_cast<uintptr_t>(f.dst[c]) % 16 == 0;
+    }
+    const long long items = vec ? g->n / 4 : g->n;
+    const dim3 grid((unsigned)std::min<long long>((items + 255) / 256, 148LL * 4), 6, 1);
+    k_frame<<<grid, 256, 0, st>>>(f, g->n, vec ? 1 : 0);
+    CUDA_TRY(cudaGetLastError());
+  }
+  return jxf_grid3d_step(g, n_steps - done, nullptr, stream);
+}
+
 int jxf_grid3d_check_error(jxf_grid3d* g, void* stream) {
   if (!g) return fail(JXF_ERR_INVALID, "null handle");
   DeviceGuard dg(g->d.device);
@@ -2194,7 +2304,8 @@ int jxf_grid3d_check_error(jxf_grid3d* g, void* stream) {
   return JXF_OK;
 }
 
-static __global__ void k_count_nonfinite(const float* f, long long n, int* count) {
+static __global__ void k_count_nonfinite(FieldPtrs6 fp, long long n, int* count) {
+  const float* f = fp.f[blockIdx.y];
   int local = 0;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
@@ -2207,7 +2318,10 @@ int jxf_grid3d_check_finite(jxf_grid3d* g, void* stream) {
   DeviceGuard dg(g->d.device);
   cudaStream_t st = (cudaStream_t)stream;
   CUDA_TRY(cudaMemsetAsync(g->d_count, 0, 4, st));
-  for (int k = 0; k < 6; ++k) k_count_nonfinite<<<592, 256, 0, st>>>(g->f[g->cur][k], g->n, g->d_count);
+  FieldPtrs6 fp;
+  for (int k = 0; k < 6; ++k) fp.f[k] = g->f[g->cur][k];
+  const unsigned blocks = (unsigned)std::min<long long>((g->n + 255) / 256, 592);
+  k_count_nonfinite<<<dim3(blocks, 6, 1), 256, 0, st>>>(fp, g->n, g->d_count);
   CUDA_TRY(cudaGetLastError());
   int h = 0;
   CUDA_TRY(cudaMemcpyAsync(&h, g->d_count, 4, cudaMemcpyDeviceToHost, st));

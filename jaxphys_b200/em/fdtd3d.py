@@ -374,6 +374,19 @@ class EMGrid3D:
                                                     nat.stream_handle()), "set_eps")
         elif self._eps_override is None and not self._materials and self._conductor is None:
             nat.check(lib.jxf_grid3d_set_eps_host(self._h, None), "set_eps")
+        elif self._eps_override is None and all(np.ndim(m.epsilon_r) == 0 and m.epsilon_r > 0
+                                               for m in self._materials):
+            # the masks go to the device as they are (a byte per cell)
+            masks = [np.ascontiguousarray(_to_numpy(m.mask).astype(bool, copy=False))
+                     for m in self._materials]
+            values = [float(m.epsilon_r) for m in self._materials]
+            if self._conductor is not None:
+                masks.append(self._conductor)
+                values.append(np.inf)
+            eps = np.array(values, dtype=np.float64)
+            ptrs = (C.c_void_p * len(masks))(*[m.ctypes.data for m in masks])
+            nat.check(lib.jxf_grid3d_set_materials(self._h, len(masks), ptrs, eps.ctypes.data),
+                      "set_materials")
         else:
             eps = np.ascontiguousarray(self.epsilon_r(), dtype=np.float64)
             nat.check(lib.jxf_grid3d_set_eps_host(self._h, eps.ctypes.data), "set_eps")
@@ -532,6 +545,37 @@ class EMGrid3D:
         if finite:
             nat.check(lib.jxf_grid3d_check_finite(self._h, nat.stream_handle()), "fields")
 
+    def _run_to_host(self, n_steps, saved, hist, stage, copy_stream, main) -> None:
+        """Run with the saved frames streamed through two device slots into
+        the pinned host tensors ``hist``."""
+        import torch
+
+        lib = nat.load()
+        st = nat.stream_handle()
+        slot_free = [None, None]
+        done = 0
+        for s, k in enumerate(saved):
+            if k + 1 > done:
+                nat.check(lib.jxf_grid3d_step(self._h, k + 1 - done, None, st), "jxf_grid3d_step")
+                done = k + 1
+            slot = s % 2
+            if slot_free[slot] is not None:
+                main.wait_event(slot_free[slot])  # its previous frame has reached the host
+            for c in range(6):
+                nat.check(lib.jxf_grid3d_get_field(self._h, c, stage[slot][c].data_ptr(), 0, st),
+                          "get_field")
+            ready = torch.cuda.Event()
+            ready.record(main)
+            copy_stream.wait_event(ready)
+            with torch.cuda.stream(copy_stream):
+                for c in range(6):
+                    hist[c][s].copy_(stage[slot][c], non_blocking=True)
+                slot_free[slot] = torch.cuda.Event()
+                slot_free[slot].record(copy_stream)
+        if n_steps > done:
+            nat.check(lib.jxf_grid3d_step(self._h, n_steps - done, None, st), "jxf_grid3d_step")
+        copy_stream.synchronize()
+
     # ---------------------------------------------------------- simulate
     def simulate(
         self,
@@ -586,7 +630,6 @@ class EMGrid3D:
             stage = [torch.empty((6,) + self.size, dtype=torch.float32, device=dev)
                      for _ in range(2)]
             copy_stream = torch.cuda.Stream(device=dev)
-            slot_free = [None, None]
         else:
             hist = [torch.empty((len(saved),) + self.size, dtype=torch.float32, device=dev)
                     for _ in COMPONENTS]
@@ -594,34 +637,12 @@ class EMGrid3D:
         main = torch.cuda.current_stream(dev)
         st = nat.stream_handle()
         self._ensure_waves(max(n_steps, 1))
-        done = 0
-        for s, k in enumerate(saved):
-            if k + 1 > done:
-                nat.check(lib.jxf_grid3d_step(self._h, k + 1 - done, None, st), "jxf_grid3d_step")
-                done = k + 1
-            if not to_host:
-                for c in range(6):
-                    nat.check(lib.jxf_grid3d_get_field(self._h, c, hist[c][s].data_ptr(), 0, st),
-                              "get_field")
-                continue
-            slot = s % 2
-            if slot_free[slot] is not None:
-                main.wait_event(slot_free[slot])  # its previous frame has reached the host
-            for c in range(6):
-                nat.check(lib.jxf_grid3d_get_field(self._h, c, stage[slot][c].data_ptr(), 0, st),
-                          "get_field")
-            ready = torch.cuda.Event()
-            ready.record(main)
-            copy_stream.wait_event(ready)
-            with torch.cuda.stream(copy_stream):
-                for c in range(6):
-                    hist[c][s].copy_(stage[slot][c], non_blocking=True)
-                slot_free[slot] = torch.cuda.Event()
-                slot_free[slot].record(copy_stream)
-        if n_steps > done:
-            nat.check(lib.jxf_grid3d_step(self._h, n_steps - done, None, st), "jxf_grid3d_step")
-        if to_host:
-            copy_stream.synchronize()
+        if not to_host:
+            ptrs = (C.c_void_p * 6)(*[h.data_ptr() for h in hist])
+            nat.check(lib.jxf_grid3d_run(self._h, max(n_steps, 0), stride, len(saved), ptrs, st),
+                      "jxf_grid3d_run")
+        else:
+            self._run_to_host(n_steps, saved, hist, stage, copy_stream, main)
         self.check(finite=True)
         t = np.array([t_start + k * dt + dt for k in saved], dtype=np.float64)
         gx = np.arange(nx) * dx
