@@ -2170,24 +2170,45 @@ int jxf_grid3d_plane(jxf_grid3d* g, int32_t comp, int32_t plane, float* buf, int
   return JXF_OK;
 }
 
+// Zeroes up to 36 arrays (both sets of fields and psi) in one launch: a reset
+// of a CPML grid was 36 memsets of 1.5 us each, 2,304 for a batch of 64.
+struct ZeroList {
+  float* p[2 * (6 + PSI_COUNT)];
+  long long n[2 * (6 + PSI_COUNT)];
+};
+static __global__ void k_zero(const __grid_constant__ ZeroList z) {
+  float* const p = z.p[blockIdx.y];
+  const long long n = z.n[blockIdx.y], n4 = n / 4;
+  const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  for (long long i = i0; i < n4; i += (long long)gridDim.x * blockDim.x)
+    reinterpret_cast<float4*>(p)[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  if (i0 < n - 4 * n4) p[4 * n4 + i0] = 0.0f;
+}
+
 int jxf_grid3d_reset(jxf_grid3d* g, void* stream) {
   if (!g) return fail(JXF_ERR_INVALID, "null handle");
   DeviceGuard dg(g->d.device);
   cudaStream_t st = (cudaStream_t)stream;
   const int sets = g->path == JXF_PATH_GENERIC ? 1 : 2;
+  const long long psi_n[3] = {(long long)g->L[0] * g->d.ny * g->d.nz,
+                              (long long)g->d.nx * g->L[1] * g->d.nz,
+                              (long long)g->d.nx * g->d.ny * g->L[2]};
+  const int axis_of[PSI_COUNT] = {1, 2, 2, 0, 0, 1, 1, 2, 2, 0, 0, 1};
+  ZeroList z{};
+  int arrays = 0;
+  long long most = 0;
+  auto add = [&](float* p, long long n) {
+    z.p[arrays] = p;
+    z.n[arrays++] = n;
+    most = std::max(most, n);
+  };
   for (int s = 0; s < sets; ++s) {
-    for (int k = 0; k < 6; ++k) CUDA_TRY(cudaMemsetAsync(g->f[s][k], 0, (size_t)g->n * 4, st));
-    if (g->mode == MODE_CPML) {
-      const size_t sz_x = (size_t)g->L[0] * g->d.ny * g->d.nz;
-      const size_t sz_y = (size_t)g->d.nx * g->L[1] * g->d.nz;
-      const size_t sz_z = (size_t)g->d.nx * g->d.ny * g->L[2];
-      const int axis_of[PSI_COUNT] = {1, 2, 2, 0, 0, 1, 1, 2, 2, 0, 0, 1};
-      for (int k = 0; k < PSI_COUNT; ++k) {
-        const size_t sz = axis_of[k] == 0 ? sz_x : (axis_of[k] == 1 ? sz_y : sz_z);
-        CUDA_TRY(cudaMemsetAsync(g->psi[s][k], 0, sz * 4, st));
-      }
-    }
+    for (int k = 0; k < 6; ++k) add(g->f[s][k], g->n);
+    for (int k = 0; k < PSI_COUNT && g->mode == MODE_CPML; ++k) add(g->psi[s][k], psi_n[axis_of[k]]);
   }
+  const unsigned blocks = (unsigned)std::min<long long>((most / 4 + 255) / 256 + 1, 148LL * 2);
+  k_zero<<<dim3(blocks, arrays, 1), 256, 0, st>>>(z);
+  CUDA_TRY(cudaGetLastError());
   g->cur = 0;
   g->step = 0;
   return JXF_OK;
