@@ -366,4 +366,27 @@ __global__ void __launch_bounds__(sweep_threads(MODE, V0), sweep_min_blocks(MODE
   sweep_block<H, MODE, V0, V1, KAPPA, CBARR>(p, s, blockIdx.y, blockIdx.x);
 }
 
+// The same pass over several grids of a batch in one launch.  Their parameters
+// ride in the launch (constant memory): read from global memory they would put
+// a dependent load in front of every block's first field load.
+constexpr int SWEEP_GROUP = 8;
+struct SweepGroup {
+  int n;
+  int end[SWEEP_GROUP];       // blocks of grids 0 .. k
+  FastDiv dblk[SWEEP_GROUP];  // divide by a grid's blocks per plane
+  Step3D p[SWEEP_GROUP];
+  SweepPlan s[SWEEP_GROUP];
+};
+template <bool H, int MODE, int V0, int V1, bool KAPPA, bool CBARR>
+__global__ void __launch_bounds__(sweep_threads(MODE, V0), sweep_min_blocks(MODE, V0))
+    k3d_sweep_group(const __grid_constant__ SweepGroup g) {
+  grid_dep_wait();
+  grid_dep_launch_dependents();
+  int k = 0;
+  while ((int)blockIdx.x >= g.end[k]) ++k;
+  const int b = (int)blockIdx.x - (k > 0 ? g.end[k - 1] : 0);
+  const int x = (int)fdiv((uint32_t)b, g.dblk[k]);
+  sweep_block<H, MODE, V0, V1, KAPPA, CBARR>(g.p[k], g.s[k], x, b - x * g.s[k].nblk);
+}
+
 }  // namespace jxf

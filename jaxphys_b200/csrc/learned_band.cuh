@@ -298,6 +298,8 @@ __global__ void __launch_bounds__(128, 5) k_band_infer(const __grid_constant__ I
   int cur_face = -1;
   bool ok = true, timed = false;
   int2 cg_next = p.cells[t0 * kTile + tid];  // (cell, grid) of the next tile, loaded a tile early
+  grid_dep_wait();  // the step's fields
+  grid_dep_launch_dependents();
   for (int t = t0; t < t1 && ok; ++t) {
     const int face = p.tile_face[t];
     const int2 cg = cg_next;
@@ -443,6 +445,8 @@ __global__ void __launch_bounds__(128, 5) k_band_infer(const __grid_constant__ I
 // stored: the fields keep the plain Yee step.
 __global__ void k_band_apply(const GridRef* grids, const int2* cells, int n, const float* xnew,
                              const int* err) {
+  grid_dep_wait();  // the corrected values
+  grid_dep_launch_dependents();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   if (__ldcg(err) != 0) return;

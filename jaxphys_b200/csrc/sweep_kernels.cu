@@ -7,9 +7,15 @@ namespace {
 
 template <int MODE, bool KAPPA, int V0, int V1>
 SweepKernels make(bool cbarr) {
+  constexpr int B = MODE == MODE_PERIODIC ? MODE_ABSORB : MODE;
   return SweepKernels{k3d_sweep<true, MODE, V0, V1, KAPPA, false>,
                       cbarr ? k3d_sweep<false, MODE, V0, V1, KAPPA, true>
                             : k3d_sweep<false, MODE, V0, V1, KAPPA, false>,
+                      // (periodic grids are not batched)
+                      MODE == MODE_PERIODIC ? nullptr : k3d_sweep_group<true, B, V0, V1, KAPPA, false>,
+                      MODE == MODE_PERIODIC ? nullptr
+                      : cbarr               ? k3d_sweep_group<false, B, V0, V1, KAPPA, true>
+                                            : k3d_sweep_group<false, B, V0, V1, KAPPA, false>,
                       V0, V1, sweep_threads(MODE, V0)};
 }
 

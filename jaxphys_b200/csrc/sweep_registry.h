@@ -8,9 +8,11 @@
 namespace jxf {
 
 using SweepKernel = void (*)(const Step3D, const SweepPlan);
+using SweepGroupKernel = void (*)(const SweepGroup);
 
 struct SweepKernels {
   SweepKernel h, e;
+  SweepGroupKernel group_h, group_e;
   int v0, v1;   // cells per thread outside / inside the z slabs
   int threads;  // per block
 };
