@@ -18,8 +18,8 @@
 #include <vector>
 
 #include "../../include/jaxphys_fdtd.h"
+#include "adjoint_registry.h"
 #include "fdtd2d_kernels.cuh"
-#include "fdtd3d_adjoint.cuh"
 #include "fdtd3d_kernels.cuh"
 #include "learned_band.cuh"
 #include "sweep_registry.h"
@@ -305,7 +305,7 @@ struct jxf_grid3d {
   size_t adj_state = 0, adj_segstate = 0;  // floats per checkpoint / per snapshot
   float* adj_ck = nullptr;
   float* adj_sg = nullptr;
-  float* adj_l = nullptr;   // lE(3n) lH(3n) lpsi(psi) db(6n) dh(6n)
+  float* adj_l = nullptr;   // lE(3n) lH(3n), two sets of lpsi
   double* adj_g = nullptr;  // dJ/dcb
   size_t adj_ck_cap = 0, adj_sg_cap = 0, adj_l_cap = 0, adj_g_cap = 0;
   // TMA selection
@@ -1098,42 +1098,61 @@ bool sweep_ok(const jxf_grid3d* g) {
          (long long)g->d.nx * g->d.ny * g->L[2] < (1LL << 31);
 }
 
-// The work split of a plane (SweepPlan) and the source lists of its blocks.
+// The work split of a plane for kernels of v0 / v1 cells per thread outside /
+// inside the z slabs.  margin: cells on the inner side of each psi slab that
+// belong to its regions too.
+SweepPlan plan_plane(const jxf_grid3d* g, int v0, int v1, int threads, int margin) {
+  const int nx = g->d.nx, ny = g->d.ny, nz = g->d.nz;
+  SweepPlan s{};
+  s.x1 = nx;
+  s.y1 = ny;
+  s.z1 = nz;
+  if (g->mode == MODE_CPML) {
+    // columns outside the z slabs start and end on 32-byte sectors: the z
+    // regions' loads and stores then share none with them (128^3, 10 layers:
+    // 24.0 us a step against 24.7 on multiples of four cells)
+    const int al = v0 > 1 ? 8 : 1;
+    int lo[3], hi[3];
+    const int n[3] = {nx, ny, nz};
+    for (int k = 0; k < 3; ++k) {
+      lo[k] = g->P[k] + margin;
+      hi[k] = n[k] - g->P[k] - margin;
+      if (k == 2) {
+        lo[k] = (lo[k] + al - 1) / al * al;
+        hi[k] = hi[k] / al * al;
+      }
+      if (g->P[k] < 0 || hi[k] <= lo[k]) lo[k] = hi[k] = 0;
+    }
+    s.x0 = lo[0];
+    s.x1 = hi[0];
+    s.y0 = lo[1];
+    s.y1 = hi[1];
+    s.z0 = lo[2];
+    s.z1 = hi[2];
+  }
+  const int slab_rows = s.y0 + ny - s.y1, mid_rows = s.y1 - s.y0;
+  const int slab_w = (s.z0 + nz - s.z1) / v1, mid_w = (s.z1 - s.z0) / v0;
+  const int rows[4] = {slab_rows, mid_rows, slab_rows, mid_rows};
+  const int w[4] = {slab_w, slab_w, mid_w, mid_w};
+  for (int i = 0; i < 4; ++i) {
+    s.r[i].w = w[i];
+    s.r[i].n = rows[i] * w[i];
+    s.r[i].nb = (s.r[i].n + threads - 1) / threads;
+    s.r[i].dw = make_fastdiv((uint32_t)std::max(w[i], 1));
+    s.nblk += s.r[i].nb;
+  }
+  return s;
+}
+
+// The work split of the step's passes and the source lists of its blocks.
 int build_sweep(jxf_grid3d* g) {
   if (g->sweep_built) return JXF_OK;
   const int nx = g->d.nx, ny = g->d.ny, nz = g->d.nz;
   const SweepKernels k = sweep_kernels(g->mode, g->kappa, g->cb != nullptr, nz);
   SweepPlan& s = g->sw;
-  s = SweepPlan{};
-  s.x1 = nx;
-  s.y1 = ny;
-  s.z1 = nz;
-  if (g->mode == MODE_CPML) {
-    s.x0 = g->P[0] < 0 ? 0 : g->P[0];
-    s.x1 = g->P[0] < 0 ? 0 : nx - g->P[0];
-    s.y0 = g->P[1] < 0 ? 0 : g->P[1];
-    s.y1 = g->P[1] < 0 ? 0 : ny - g->P[1];
-    // columns outside the z slabs start and end on 32-byte sectors: the z
-    // regions' loads and stores then share none with them (128^3, 10 layers:
-    // 24.0 us a step against 24.7 on multiples of four cells)
-    const int al = k.v0 > 1 ? 8 : 1;
-    s.z0 = g->P[2] < 0 ? 0 : (g->P[2] + al - 1) / al * al;
-    s.z1 = g->P[2] < 0 ? 0 : (nz - g->P[2]) / al * al;
-    if (s.z1 <= s.z0) s.z0 = s.z1 = 0;
-  }
-  const int slab_rows = s.y0 + ny - s.y1, mid_rows = s.y1 - s.y0;
-  const int slab_w = (s.z0 + nz - s.z1) / k.v1, mid_w = (s.z1 - s.z0) / k.v0;
-  const int rows[4] = {slab_rows, mid_rows, slab_rows, mid_rows};
-  const int w[4] = {slab_w, slab_w, mid_w, mid_w};
-  int base[4];
-  for (int i = 0; i < 4; ++i) {
-    s.r[i].w = w[i];
-    s.r[i].n = rows[i] * w[i];
-    s.r[i].nb = (s.r[i].n + k.threads - 1) / k.threads;
-    s.r[i].dw = make_fastdiv((uint32_t)std::max(w[i], 1));
-    base[i] = s.nblk;
-    s.nblk += s.r[i].nb;
-  }
+  s = plan_plane(g, k.v0, k.v1, k.threads, 0);
+  int base[4] = {0, 0, 0, 0};
+  for (int i = 1; i < 4; ++i) base[i] = base[i - 1] + s.r[i - 1].nb;
   std::vector<SrcCell> cells;
   std::vector<SrcTerm> terms;
   group_sources(g, cells, terms);
@@ -1181,8 +1200,9 @@ bool sweep_records(const jxf_grid3d* g, bool band) {
 
 // One in-place step on buffer set `set` (p.probe_out: row of the state before
 // it, or null; row: row of the state after it, whose H components the E pass
-// records, or null).
-int launch_sweep(jxf_grid3d* g, Step3D& p, int set, float* row, bool sources, cudaStream_t st) {
+// records, or null; snap: where the E pass leaves H and the E psi, or null).
+int launch_sweep(jxf_grid3d* g, Step3D& p, int set, float* row, bool sources, cudaStream_t st,
+                 const SweepSnap* snap = nullptr) {
   const SweepKernels k = sweep_kernels(g->mode, g->kappa, g->cb != nullptr, g->d.nz);
   set_io(g, p, set, set);
   SweepPlan s = g->sw;
@@ -1199,13 +1219,17 @@ int launch_sweep(jxf_grid3d* g, Step3D& p, int set, float* row, bool sources, cu
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = attr;
     lc.numAttrs = g->use_pdl ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelEx(&lc, half == 0 ? k.h : k.e, p, s);
+    auto go = [&] {
+      if (half == 1 && snap) return cudaLaunchKernelEx(&lc, k.snap_e, p, s, *snap);
+      return cudaLaunchKernelEx(&lc, half == 0 ? k.h : k.e, p, s);
+    };
+    cudaError_t e = go();
     if (e != cudaSuccess && g->use_pdl) {
       // stream without programmatic serialization support: launch in order
       (void)cudaGetLastError();
       g->use_pdl = false;
       lc.numAttrs = 0;
-      e = cudaLaunchKernelEx(&lc, half == 0 ? k.h : k.e, p, s);
+      e = go();
     }
     if (e != cudaSuccess)
       return fail(JXF_ERR_CUDA, "step kernel launch failed: %s", cudaGetErrorString(e));
@@ -1941,6 +1965,18 @@ static int gather_probes(jxf_grid3d* g, int set, float* out, cudaStream_t st) {
   return JXF_OK;
 }
 
+static int check_waves3d(const jxf_grid3d* g, long long n_steps) {
+  if (g->src_cell.empty()) return JXF_OK;
+  int max_w = 0;
+  for (int w : g->src_wave) max_w = std::max(max_w, w);
+  if (max_w >= g->n_waves)
+    return fail(JXF_ERR_INVALID, "source wave id %d has no waveform row", max_w);
+  if (g->step + n_steps > g->wave_len)
+    return fail(JXF_ERR_INVALID, "waveform table covers %lld steps, need %lld", g->wave_len,
+                g->step + n_steps);
+  return JXF_OK;
+}
+
 int jxf_grid3d_step(jxf_grid3d* g, int32_t n_steps, float* probe_out, void* stream) {
   if (!g) return fail(JXF_ERR_INVALID, "null handle");
   if (g->slab && g->path != JXF_PATH_TMA)
@@ -1951,15 +1987,7 @@ int jxf_grid3d_step(jxf_grid3d* g, int32_t n_steps, float* probe_out, void* stre
                 "exchanged between steps)");
   if (n_steps < 0) return fail(JXF_ERR_INVALID, "n_steps must be >= 0");
   if (n_steps == 0) return JXF_OK;
-  if (!g->src_cell.empty()) {
-    int max_w = 0;
-    for (int w : g->src_wave) max_w = std::max(max_w, w);
-    if (max_w >= g->n_waves)
-      return fail(JXF_ERR_INVALID, "source wave id %d has no waveform row", max_w);
-    if (g->step + n_steps > g->wave_len)
-      return fail(JXF_ERR_INVALID, "waveform table covers %lld steps, need %lld", g->wave_len,
-                  g->step + n_steps);
-  }
+  TRY(check_waves3d(g, n_steps));
   DeviceGuard dg(g->d.device);
   cudaStream_t st = (cudaStream_t)stream;
   Step3D p = base_params(g);
@@ -4386,6 +4414,9 @@ size_t psi_size(const jxf_grid3d* g, int id) {
   return (size_t)g->d.nx * g->d.ny * g->L[2];
 }
 
+// arrays of a snapshot start on 16 bytes
+size_t pad4(size_t n) { return (n + 3) / 4 * 4; }
+
 template <class T>
 int ensure_buf(T** p, size_t* cap, size_t count, int64_t* tally) {
   if (*cap >= count && *p) return JXF_OK;
@@ -4474,9 +4505,9 @@ extern "C" int jxf_grid3d_adjoint_forward(jxf_grid3d* g, int32_t n_steps,
   const int K = checkpoint_every > 0 ? checkpoint_every
                                      : std::max(1, (int)std::ceil(std::sqrt((double)n_steps)));
   const int nseg = (n_steps + K - 1) / K;
-  size_t state = 6 * (size_t)g->n, segstate = 3 * (size_t)g->n;
+  size_t state = 6 * (size_t)g->n, segstate = 3 * pad4((size_t)g->n);
   for (int k = 0; k < PSI_COUNT; ++k) state += psi_size(g, k);
-  for (int k = PSI_EXY; k < PSI_COUNT; ++k) segstate += psi_size(g, k);
+  for (int k = PSI_EXY; k < PSI_COUNT; ++k) segstate += pad4(psi_size(g, k));
   TRY(ensure_buf(&g->adj_ck, &g->adj_ck_cap, state * nseg, &g->bytes));
   TRY(jxf_grid3d_reset(g, stream));
   const int np = g->n_probes;
@@ -4505,18 +4536,16 @@ extern "C" int jxf_grid3d_adjoint_backward(jxf_grid3d* g, const float* probe_gra
   size_t psi_tot = 0;
   for (int k = 0; k < PSI_COUNT; ++k) psi_tot += psi_size(g, k);
   TRY(ensure_buf(&g->adj_sg, &g->adj_sg_cap, g->adj_segstate * K, &g->bytes));
-  TRY(ensure_buf(&g->adj_l, &g->adj_l_cap, 18 * n + psi_tot, &g->bytes));
+  // adjoint fields, and two sets of adjoint psi
+  TRY(ensure_buf(&g->adj_l, &g->adj_l_cap, 6 * n + 2 * psi_tot, &g->bytes));
   TRY(ensure_buf(&g->adj_g, &g->adj_g_cap, n, &g->bytes));
-  CUDA_TRY(cudaMemsetAsync(g->adj_l, 0, (18 * n + psi_tot) * 4, st));
+  CUDA_TRY(cudaMemsetAsync(g->adj_l, 0, (6 * n + 2 * psi_tot) * 4, st));
   CUDA_TRY(cudaMemsetAsync(g->adj_g, 0, n * 8, st));
 
   Adj3D a{};
   a.nx = g->d.nx;
   a.ny = g->d.ny;
   a.nz = g->d.nz;
-  a.div_nz = make_fastdiv((uint32_t)g->d.nz);
-  a.div_ny = make_fastdiv((uint32_t)g->d.ny);
-  a.idx32 = ((long long)g->d.nx * g->d.ny * g->d.nz) < (1ll << 32) ? 1 : 0;
   a.a = (float)g->coef_h;
   a.cb_const = (float)g->coef_e;
   a.cb = g->cb;
@@ -4534,70 +4563,94 @@ extern "C" int jxf_grid3d_adjoint_backward(jxf_grid3d* g, const float* probe_gra
     lam.f[c] = a.lE[c];
     lam.f[3 + c] = a.lH[c];
   }
-  {
-    size_t off = 6 * n;
+  float* lpsi[2][PSI_COUNT];
+  size_t psi_off = 6 * n;
+  for (int s = 0; s < 2; ++s)
     for (int k = 0; k < PSI_COUNT; ++k) {
-      a.lpsi[k] = psi_size(g, k) ? lp + off : nullptr;
-      off += psi_size(g, k);
+      lpsi[s][k] = lp + psi_off;
+      psi_off += psi_size(g, k);
     }
-    for (int k = 0; k < 6; ++k) {
-      a.db[k] = lp + off + k * n;
-      a.dh[k] = lp + off + (6 + k) * n;
-    }
-  }
   a.gcb = g->adj_g;
   const int threads = 256;
   const int blocks = (int)std::min<long long>(((long long)n + threads - 1) / threads, 148LL * 16);
   const int np = g->n_probes;
+  const AdjKernels ak = adj_kernels(g->mode, g->kappa, g->cb != nullptr, g->d.nz);
+  const SweepPlan plan = plan_plane(g, ak.v, ak.v, ADJ_THREADS, 1);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t lc{};
+  lc.stream = st;
+  lc.attrs = attr;
+  lc.numAttrs = g->use_pdl ? 1 : 0;
+  // segments recomputed on the in-place passes leave their snapshots from the
+  // E pass; other launches (and a band, which corrects the state) are copied
+  if (g->path == JXF_PATH_TMA) TRY(ensure_tma_ready(g, st));
+  const bool in_pass =
+      (g->sweep || (g->path == JXF_PATH_GENERIC && sweep_ok(g))) && !g->band.band;
+  if (in_pass) TRY(build_sweep(g));
+  Step3D sp = base_params(g);
 
+  int set = 0;  // adjoint psi before the step
   for (int s = g->adj_nseg - 1; s >= 0; --s) {
     const int start = s * K, len = std::min(K, N - start);
     // recompute the segment, keeping (H, psiE) after every step
     TRY(ckpt_copy(g, g->adj_ck + (size_t)s * g->adj_state, false, st));
     g->step = start;
+    TRY(check_waves3d(g, len));
     for (int k = 0; k < len; ++k) {
-      TRY(jxf_grid3d_step(g, 1, nullptr, stream));
-      float* slot = g->adj_sg + (size_t)k * g->adj_segstate;
-      size_t off = 0;
-      CopyBatch cb;
+      SweepSnap sn{};
+      size_t off = (size_t)k * g->adj_segstate;
       for (int c = 0; c < 3; ++c) {
-        cb.add(slot + off, g->f[g->cur][3 + c], n);
-        off += n;
+        sn.h[c] = g->adj_sg + off;
+        off += pad4(n);
       }
-      for (int q = PSI_EXY; q < PSI_COUNT; ++q) {
-        const size_t sz = psi_size(g, q);
-        cb.add(slot + off, g->psi[g->cur][q], sz);
-        off += sz;
+      for (int q = 0; q < 6; ++q) {
+        sn.psi[q] = g->adj_sg + off;
+        off += pad4(psi_size(g, PSI_EXY + q));
       }
+      if (in_pass) {
+        sp.step = g->step;
+        sp.probe_out = nullptr;
+        TRY(launch_sweep(g, sp, g->cur, nullptr, !g->src_cell.empty(), st, &sn));
+        g->step++;
+        continue;
+      }
+      TRY(jxf_grid3d_step(g, 1, nullptr, stream));
+      CopyBatch cb;
+      for (int c = 0; c < 3; ++c) cb.add(sn.h[c], g->f[g->cur][3 + c], n);
+      for (int q = 0; q < 6; ++q)
+        cb.add(sn.psi[q], g->psi[g->cur][PSI_EXY + q], psi_size(g, PSI_EXY + q));
       TRY(cb.launch(st));
     }
     // adjoint steps, last to first
     for (int k = len - 1; k >= 0; --k) {
       const int step_n = start + k;
       if (np > 0) {
-        k3a_seed<<<1, 32, 0, st>>>(lam, g->d_probe_cell, g->d_probe_comp, np,
-                                   probe_grad + (size_t)step_n * np);
+        lc.gridDim = dim3(1, 1, 1);
+        lc.blockDim = dim3(32, 1, 1);
+        CUDA_TRY(cudaLaunchKernelEx(&lc, k3a_seed, lam, (const long long*)g->d_probe_cell,
+                                    (const int*)g->d_probe_comp, np,
+                                    probe_grad + (size_t)step_n * np));
       }
-      const float* slot = g->adj_sg + (size_t)k * g->adj_segstate;
-      size_t off = 0;
+      size_t off = (size_t)k * g->adj_segstate;
       for (int c = 0; c < 3; ++c) {
-        a.fh[c] = slot + off;
-        off += n;
+        a.fh[c] = g->adj_sg + off;
+        off += pad4(n);
       }
-      for (int q = PSI_EXY; q < PSI_COUNT; ++q) {
-        const size_t sz = psi_size(g, q);
-        a.fpsiE[q - PSI_EXY] = sz ? slot + off : nullptr;
-        off += sz;
+      for (int q = 0; q < 6; ++q) {
+        a.fpsiE[q] = g->adj_sg + off;
+        off += pad4(psi_size(g, PSI_EXY + q));
       }
-      if (g->mode == MODE_CPML) {
-        k3a_e<MODE_CPML><<<blocks, threads, 0, st>>>(a);
-        k3a_h<MODE_CPML><<<blocks, threads, 0, st>>>(a);
-      } else {
-        k3a_e<MODE_ABSORB><<<blocks, threads, 0, st>>>(a);
-        k3a_h<MODE_ABSORB><<<blocks, threads, 0, st>>>(a);
+      for (int q = 0; q < PSI_COUNT; ++q) {
+        a.pml.in[q] = lpsi[set][q];
+        a.pml.out[q] = lpsi[set ^ 1][q];
       }
-      k3a_e2<<<blocks, threads, 0, st>>>(a);
-      CUDA_TRY(cudaGetLastError());
+      set ^= 1;
+      lc.gridDim = dim3(plan.nblk, std::min(g->d.nx, 65535), 1);
+      lc.blockDim = dim3(ADJ_THREADS, 1, 1);
+      CUDA_TRY(cudaLaunchKernelEx(&lc, ak.e, a, plan));
+      CUDA_TRY(cudaLaunchKernelEx(&lc, ak.h, a, plan));
     }
   }
   k3a_finish<<<blocks, threads, 0, st>>>(g->adj_g, g->cb, (float)g->coef_e, g->coef_e, grad_eps,

@@ -7,206 +7,362 @@
 //   psiE' = bE psiE + cE G(H')                      G: backward differences
 //   E'    = damp (E + cb (kE G(H') + S psiE')) + src
 // Its transpose, applied to the adjoint (Ebar', Hbar', psibar') of the
-// step's outputs, gives the adjoint of its inputs:
-//   k3a_e : X = kE G(H') + S psiE' from the stored forward state;
-//           dJ/dcb += damp Ebar' X (FP64); Xbar = cb damp Ebar';
-//           psibarE' += S^T Xbar;  dbarE = kE^T Xbar + cE psibarE';
-//           psibarE = bE psibarE';  Ebar = damp Ebar'
-//   k3a_h : Hbar' += G^T dbarE (gather);  Ybar = -a Hbar';
-//           psibarH' += S^T Ybar;  dbarH = kH^T Ybar + cH psibarH';
-//           psibarH = bH psibarH';  Hbar = Hbar'
-//   k3a_e2: Ebar += D^T dbarH (gather)
+// step's outputs, gives the adjoint of its inputs, in two passes:
+//   k3a_pass<true>:  Xbar = cb damp Ebar';  psibarE' += S^T Xbar;
+//                    dbarE = kE^T Xbar + cE psibarE';  psibarE = bE psibarE';
+//                    Hbar += G^T dbarE (gather from the cell and its upper
+//                    neighbours);  dJ/dcb += damp Ebar' X (FP64) with
+//                    X = kE G(H') + S psiE' from the stored forward state
+//   k3a_pass<false>: Ybar = -a Hbar;  psibarH' += S^T Ybar;
+//                    dbarH = kH^T Ybar + cH psibarH';  psibarH = bH psibarH';
+//                    Ebar = damp Ebar' + D^T dbarH (cell and lower neighbours)
 // Cells outside a component's update range are the identity (no curl term),
 // exactly as in the forward step.  Adjoint fields are FP32; dJ/dcb is
 // accumulated in FP64.
+//
+// The difference adjoints dbarE and dbarH are formed where they are gathered,
+// from Ebar (Hbar) and psibar of the cell and its three neighbours, instead of
+// going through twelve arrays: 3 launches and about 190 bytes per cell and
+// step became 2 launches and 130, on a working set (fields, dJ/dcb, psi: 60 MB
+// at 96^3) that stays in the L2.  A pass reads one psi set and writes the
+// other, because a neighbour's thread reads the value from before the step.
+// 96^3, 10-layer CPML, per step: 80 us before, 25 now.
 #pragma once
 
-#include "fdtd3d_kernels.cuh"
+#include "fdtd3d_sweep.cuh"
 
 namespace jxf {
 
-// db arrays of the E phase (adjoint of the H differences used by E):
-//   0: Ex / dHz/dy   1: Ex / dHy/dz   2: Ey / dHx/dz
-//   3: Ey / dHz/dx   4: Ez / dHy/dx   5: Ez / dHx/dy
-// dh arrays of the H phase (adjoint of the E differences used by H):
-//   0: Hx / dEz/dy   1: Hx / dEy/dz   2: Hy / dEx/dz
-//   3: Hy / dEz/dx   4: Hz / dEy/dx   5: Hz / dEx/dy
+constexpr int ADJ_THREADS = 128;
+
 struct Adj3D {
   int nx, ny, nz;
   float a, cb_const;
   const float* cb;
   const float* damp[3];
-  CpmlDev pml;                // tables, slab maps (in/out unused)
-  const float* fh[3];         // forward H^{n+1/2} after the step
-  const float* fpsiE[6];      // forward psi (EXY..EZY) after the step, slab layout
-  float* lE[3];               // adjoint of E
-  float* lH[3];               // adjoint of H
-  float* lpsi[PSI_COUNT];     // adjoint of psi, slab layout
-  float* db[6];
-  float* dh[6];
-  double* gcb;                // dJ/dcb accumulator
-  FastDiv div_nz, div_ny;     // index decode (idx32: nx ny nz < 2^32)
-  int idx32;
+  CpmlDev pml;            // tables, slab maps; in / out: adjoint of psi
+  const float* fh[3];     // forward H^{n+1/2} after the step
+  const float* fpsiE[6];  // forward psi (EXY..EZY) after the step, slab layout
+  float* lE[3];           // adjoint of E
+  float* lH[3];           // adjoint of H
+  double* gcb;            // dJ/dcb accumulator
 };
 
-// psi adjoint through one term: tot = carried + u; new carried = b * tot;
-// returns c * tot (the term's contribution to the difference adjoint).
-__device__ __forceinline__ float adj_psi(float* lp, long long idx, float b, float c, float u) {
-  const float tot = lp[idx] + u;
-  lp[idx] = b * tot;
-  return c * tot;
+// Adjoint of one difference of a component's curl: the component's adjoint u
+// (with the term's sign) through 1/kappa and the psi recurrence.
+template <bool KAPPA>
+__device__ __forceinline__ float adj_diff(bool slab, float u, float ik, float c, float psi) {
+  const float d = KAPPA ? ik * u : u;
+  return slab ? d + c * (psi + u) : d;
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(256) k3a_e(const __grid_constant__ Adj3D p) {
+// One thread's cells (x, y, z0 .. z0+V-1).  P1: the pass over the E adjoint
+// (updates Hbar and dJ/dcb, neighbours one up); else the pass over the H
+// adjoint (updates Ebar, neighbours one down).  XS / YS / ZS (CPML): a cell or
+// its neighbour may lie in that axis's psi slab.  Differences by component and
+// axis: 0 x/y, 1 x/z, 2 y/z, 3 y/x, 4 z/x, 5 z/y.
+template <bool P1, int MODE, int V, bool KAPPA, bool CBARR, bool XS, bool YS, bool ZS>
+__device__ __forceinline__ void adj_cells(const Adj3D& p, int x, int y, int z0) {
+  constexpr bool CP = MODE == MODE_CPML;
+  constexpr bool DAMP = MODE == MODE_ABSORB;
+  constexpr int S = P1 ? 1 : -1;  // direction of the neighbours
   const int nx = p.nx, ny = p.ny, nz = p.nz;
-  const long long n = (long long)nx * ny * nz;
-  constexpr bool CP = (MODE == MODE_CPML);
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    int x, y, z;
-    decode_cell(i, nz, ny, p.idx32 != 0, p.div_nz, p.div_ny, x, y, z);
-    const float cb = p.cb ? p.cb[i] : p.cb_const;
-    float damp = 1.0f;
-    if (MODE == MODE_ABSORB)
-      damp = (p.damp[0][x] * p.damp[1][y]) * p.damp[2][z];
-    int im = -1, jm = -1, km = -1;
-    AxisCoef cx{}, cy{}, cz{};
-    if (CP) {
-      im = slab_map(x, nx, p.pml.P[0]);
-      jm = slab_map(y, ny, p.pml.P[1]);
-      km = slab_map(z, nz, p.pml.P[2]);
-      cx = axis_coef(p.pml, 0, x);
-      cy = axis_coef(p.pml, 1, y);
-      cz = axis_coef(p.pml, 2, z);
+  const int plane = ny * nz;
+  const long long idx = (long long)x * plane + (y * nz + z0);
+  // update conditions of the components, and which neighbours exist
+  const bool okx = (CP && !XS) || (P1 ? x >= 1 : x < nx - 1);
+  const bool oky = (CP && !YS) || (P1 ? y >= 1 : y < ny - 1);
+  const bool ex = (CP && !XS) || (P1 ? x < nx - 1 : x >= 1);
+  const bool ey = (CP && !YS) || (P1 ? y < ny - 1 : y >= 1);
+  const int zn = P1 ? z0 + V : z0 - 1;  // z neighbour of the vector's end
+  const bool ez = (CP && !ZS) || (P1 ? zn < nz : zn >= 0);
+  // (a neighbour that does not exist is read at the cell and not used)
+  const long long ix = ex ? idx + S * plane : idx;
+  const long long iy = ey ? idx + S * nz : idx;
+  const long long iz = ez ? (P1 ? idx + V : idx - 1) : idx;
+  float* const* const A = P1 ? p.lE : p.lH;
+  float* const* const G = P1 ? p.lH : p.lE;
+  const VecF<V> a0 = load_v<V>(A[0] + idx), a1 = load_v<V>(A[1] + idx), a2 = load_v<V>(A[2] + idx);
+  const VecF<V> a0y = load_v<V>(A[0] + iy), a2y = load_v<V>(A[2] + iy);
+  const VecF<V> a1x = load_v<V>(A[1] + ix), a2x = load_v<V>(A[2] + ix);
+  const float a0z = A[0][iz], a1z = A[1][iz];
+  VecF<V> g0 = load_v<V>(G[0] + idx), g1 = load_v<V>(G[1] + idx), g2 = load_v<V>(G[2] + idx);
+  // component adjoint = weight * field adjoint
+  VecF<V> w, wx, wy;
+  float wz = P1 ? p.cb_const : -p.a;
+#pragma unroll
+  for (int k = 0; k < V; ++k) w.v[k] = wx.v[k] = wy.v[k] = wz;
+  if (P1 && CBARR) {
+    w = load_v<V>(p.cb + idx);
+    wx = load_v<V>(p.cb + ix);
+    wy = load_v<V>(p.cb + iy);
+    wz = p.cb[iz];
+  }
+  VecF<V> damp;
+#pragma unroll
+  for (int k = 0; k < V; ++k) damp.v[k] = 1.0f;
+  if (DAMP) {
+    const int xn = ex ? x + S : x, yn = ey ? y + S : y;
+    const float dx = __ldg(p.damp[0] + x), dy = __ldg(p.damp[1] + y);
+    const float dxn = __ldg(p.damp[0] + xn), dyn = __ldg(p.damp[1] + yn);
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      const float dz = __ldg(p.damp[2] + z0 + k);
+      damp.v[k] = (dx * dy) * dz;
+      if (P1) {
+        w.v[k] *= damp.v[k];
+        wx.v[k] *= (dxn * dy) * dz;
+        wy.v[k] *= (dx * dyn) * dz;
+      }
     }
-    const long long ix = xs_index(im, y, z, ny, nz);
-    const long long iy = ys_index(x, jm, z, p.pml.L[1], nz);
-    const long long iz = zs_index(x, y, km, ny, p.pml.L[2]);
-    const float* hx = p.fh[0];
-    const float* hy = p.fh[1];
-    const float* hz = p.fh[2];
-    double g = 0.0;
-    float d[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    // one E component: terms (axis a1 with diff d1, slab s1, psi id q1) and
-    // (axis a2, d2, s2, q2); X = (ik1 d1 - ik2 d2) + (psi1' - psi2')
-    auto comp = [&](int c, float d1, float d2, bool s1, bool s2, int q1, int q2, long long o1,
-                    long long o2, const AxisCoef& k1, const AxisCoef& k2, int out1, int out2) {
-      const float eb = p.lE[c][i];
-      float X;
-      if (CP && (s1 || s2)) {
-        const float p1 = s1 ? p.fpsiE[q1 - PSI_EXY][o1] : 0.0f;
-        const float p2 = s2 ? p.fpsiE[q2 - PSI_EXY][o2] : 0.0f;
-        X = (k1.ike * d1 - k2.ike * d2) + (p1 - p2);
-      } else {
-        X = d1 - d2;
+    if (P1) wz *= (dx * dy) * __ldg(p.damp[2] + (ez ? zn : z0));
+  }
+  // forward H of the curl (dJ/dcb)
+  VecF<V> f0, f1, f2, f0y, f2y, f1x, f2x;
+  float f0z = 0.0f, f1z = 0.0f;
+  double gc[V];
+  if (P1) {
+    const long long jx = okx ? idx - plane : idx, jy = oky ? idx - nz : idx;
+    const long long jz = (CP && !ZS) || z0 >= 1 ? idx - 1 : idx;
+    f0 = load_v<V>(p.fh[0] + idx);
+    f1 = load_v<V>(p.fh[1] + idx);
+    f2 = load_v<V>(p.fh[2] + idx);
+    f0y = load_v<V>(p.fh[0] + jy);
+    f2y = load_v<V>(p.fh[2] + jy);
+    f1x = load_v<V>(p.fh[1] + jx);
+    f2x = load_v<V>(p.fh[2] + jx);
+    f0z = p.fh[0][jz];
+    f1z = p.fh[1][jz];
+    if constexpr (V == 2) {
+      const double2 t = *reinterpret_cast<const double2*>(p.gcb + idx);
+      gc[0] = t.x;
+      gc[1] = t.y;
+    } else {
+      gc[0] = p.gcb[idx];
+    }
+  }
+  // psi of the cell and its neighbours, coefficients of their positions
+  constexpr int Q = P1 ? PSI_EXY : PSI_HXY;
+  constexpr int QXY = Q, QXZ = Q + 1, QYZ = Q + 2, QYX = Q + 3, QZX = Q + 4, QZY = Q + 5;
+  constexpr int TB = P1 ? TAB_BE : TAB_BH, TC = P1 ? TAB_CE : TAB_CH, TK = P1 ? TAB_IKE : TAB_IKH;
+  VecF<V> zero;
+#pragma unroll
+  for (int k = 0; k < V; ++k) zero.v[k] = 0.0f;
+  VecF<V> qyx = zero, qzx = zero, qxy = zero, qzy = zero;      // of the cell
+  VecF<V> nyx = zero, nzx = zero, nxy = zero, nzy = zero;      // of the x / y neighbour
+  VecF<V> pxy = zero, pzy = zero, pyx = zero, pzx = zero;      // forward psi
+  float qxz[V], qyz[V], nxz = 0.0f, nyz = 0.0f, pxz[V], pyz[V];
+  float xc = 0, xk = 1, xcn = 0, xkn = 1, xb = 0, yc = 0, yk = 1, ycn = 0, ykn = 1, yb = 0;
+  float zb[V], zc[V], zk[V], zcn = 0.0f, zkn = 1.0f;
+  bool sx = false, sxn = false, sy = false, syn = false, sz[V], szn = false;
+  long long ox = 0, oy = 0, oz = 0;
+  int km[V];
+#pragma unroll
+  for (int k = 0; k < V; ++k) {
+    qxz[k] = qyz[k] = pxz[k] = pyz[k] = zb[k] = zc[k] = 0.0f;
+    zk[k] = 1.0f;
+    sz[k] = false;
+    km[k] = -1;
+  }
+  if (XS) {
+    const int im = slab_map(x, nx, p.pml.P[0]);
+    const int imn = ex ? slab_map(x + S, nx, p.pml.P[0]) : -1;
+    sx = im >= 0;
+    sxn = imn >= 0;
+    if (sx) {
+      ox = ((long long)im * ny + y) * nz + z0;
+      xb = __ldg(p.pml.tab[0][TB] + x);
+      xc = __ldg(p.pml.tab[0][TC] + x);
+      if (KAPPA) xk = __ldg(p.pml.tab[0][TK] + x);
+      qyx = load_v<V>(p.pml.in[QYX] + ox);
+      qzx = load_v<V>(p.pml.in[QZX] + ox);
+      if (P1) {
+        pyx = load_v<V>(p.fpsiE[PSI_EYX - PSI_EXY] + ox);
+        pzx = load_v<V>(p.fpsiE[PSI_EZX - PSI_EXY] + ox);
       }
-      g += (double)eb * (double)damp * (double)X;
-      const float xb = cb * damp * eb;
-      float u1 = xb, u2 = -xb;  // adjoints of ik*d terms before ik
-      if (CP && (s1 || s2)) {
-        const float c1 = s1 ? adj_psi(p.lpsi[q1], o1, k1.be, k1.ce, xb) : 0.0f;
-        const float c2 = s2 ? adj_psi(p.lpsi[q2], o2, k2.be, k2.ce, -xb) : 0.0f;
-        u1 = k1.ike * xb + c1;
-        u2 = -k2.ike * xb + c2;
+    }
+    if (sxn) {
+      const long long o = ((long long)imn * ny + y) * nz + z0;
+      xcn = __ldg(p.pml.tab[0][TC] + x + S);
+      if (KAPPA) xkn = __ldg(p.pml.tab[0][TK] + x + S);
+      nyx = load_v<V>(p.pml.in[QYX] + o);
+      nzx = load_v<V>(p.pml.in[QZX] + o);
+    }
+  }
+  if (YS) {
+    const int jm = slab_map(y, ny, p.pml.P[1]);
+    const int jmn = ey ? slab_map(y + S, ny, p.pml.P[1]) : -1;
+    sy = jm >= 0;
+    syn = jmn >= 0;
+    if (sy) {
+      oy = ((long long)x * p.pml.L[1] + jm) * nz + z0;
+      yb = __ldg(p.pml.tab[1][TB] + y);
+      yc = __ldg(p.pml.tab[1][TC] + y);
+      if (KAPPA) yk = __ldg(p.pml.tab[1][TK] + y);
+      qxy = load_v<V>(p.pml.in[QXY] + oy);
+      qzy = load_v<V>(p.pml.in[QZY] + oy);
+      if (P1) {
+        pxy = load_v<V>(p.fpsiE[PSI_EXY - PSI_EXY] + oy);
+        pzy = load_v<V>(p.fpsiE[PSI_EZY - PSI_EXY] + oy);
       }
-      d[out1] = u1;
-      d[out2] = u2;
-    };
-    if (y >= 1 && z >= 1)  // Ex: dHz/dy - dHy/dz
-      comp(0, hz[i] - hz[i - nz], hy[i] - hy[i - 1], jm >= 0, km >= 0, PSI_EXY, PSI_EXZ, iy, iz,
-           cy, cz, 0, 1);
-    if (x >= 1 && z >= 1)  // Ey: dHx/dz - dHz/dx
-      comp(1, hx[i] - hx[i - 1], hz[i] - hz[i - (long long)ny * nz], km >= 0, im >= 0, PSI_EYZ,
-           PSI_EYX, iz, ix, cz, cx, 2, 3);
-    if (x >= 1 && y >= 1)  // Ez: dHy/dx - dHx/dy
-      comp(2, hy[i] - hy[i - (long long)ny * nz], hx[i] - hx[i - nz], im >= 0, jm >= 0, PSI_EZX,
-           PSI_EZY, ix, iy, cx, cy, 4, 5);
-    for (int k = 0; k < 6; ++k) p.db[k][i] = d[k];
-    if (g != 0.0) p.gcb[i] += g;
-    if (MODE == MODE_ABSORB)
-      for (int c = 0; c < 3; ++c) p.lE[c][i] = damp * p.lE[c][i];
+    }
+    if (syn) {
+      const long long o = ((long long)x * p.pml.L[1] + jmn) * nz + z0;
+      ycn = __ldg(p.pml.tab[1][TC] + y + S);
+      if (KAPPA) ykn = __ldg(p.pml.tab[1][TK] + y + S);
+      nxy = load_v<V>(p.pml.in[QXY] + o);
+      nzy = load_v<V>(p.pml.in[QZY] + o);
+    }
+  }
+  if (ZS) {
+    oz = ((long long)x * ny + y) * p.pml.L[2];
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      km[k] = slab_map(z0 + k, nz, p.pml.P[2]);
+      sz[k] = km[k] >= 0;
+      if (sz[k]) {
+        zb[k] = __ldg(p.pml.tab[2][TB] + z0 + k);
+        zc[k] = __ldg(p.pml.tab[2][TC] + z0 + k);
+        if (KAPPA) zk[k] = __ldg(p.pml.tab[2][TK] + z0 + k);
+        qxz[k] = p.pml.in[QXZ][oz + km[k]];
+        qyz[k] = p.pml.in[QYZ][oz + km[k]];
+        if (P1) {
+          pxz[k] = p.fpsiE[PSI_EXZ - PSI_EXY][oz + km[k]];
+          pyz[k] = p.fpsiE[PSI_EYZ - PSI_EXY][oz + km[k]];
+        }
+      }
+    }
+    const int kn = ez ? slab_map(zn, nz, p.pml.P[2]) : -1;
+    szn = kn >= 0;
+    if (szn) {
+      zcn = __ldg(p.pml.tab[2][TC] + zn);
+      if (KAPPA) zkn = __ldg(p.pml.tab[2][TK] + zn);
+      nxz = p.pml.in[QXZ][oz + kn];
+      nyz = p.pml.in[QYZ][oz + kn];
+    }
+  }
+
+  // z differences of the vector's cells and, at the end the neighbour is on,
+  // of the cell beyond
+  float d1[V + 1], d2[V + 1];
+  constexpr int B = P1 ? 0 : 1;  // cell k is entry k + B, the neighbour the other end
+  constexpr int E = P1 ? V : 0;
+  d1[E] = ez && oky ? adj_diff<KAPPA>(szn, -(wz * a0z), zkn, zcn, nxz) : 0.0f;
+  d2[E] = ez && okx ? adj_diff<KAPPA>(szn, wz * a1z, zkn, zcn, nyz) : 0.0f;
+  float d0[V], d3[V], d4[V], d5[V];
+#pragma unroll
+  for (int k = 0; k < V; ++k) {
+    const int z = z0 + k;
+    const bool okz = (CP && !ZS) || (P1 ? z >= 1 : z < nz - 1);
+    const bool u0 = oky && okz, u1 = okx && okz, u2 = okx && oky;
+    const float x0 = w.v[k] * a0.v[k], x1 = w.v[k] * a1.v[k], x2 = w.v[k] * a2.v[k];
+    d0[k] = u0 ? adj_diff<KAPPA>(sy, x0, yk, yc, qxy.v[k]) : 0.0f;
+    d1[k + B] = u0 ? adj_diff<KAPPA>(sz[k], -x0, zk[k], zc[k], qxz[k]) : 0.0f;
+    d2[k + B] = u1 ? adj_diff<KAPPA>(sz[k], x1, zk[k], zc[k], qyz[k]) : 0.0f;
+    d3[k] = u1 ? adj_diff<KAPPA>(sx, -x1, xk, xc, qyx.v[k]) : 0.0f;
+    d4[k] = u2 ? adj_diff<KAPPA>(sx, x2, xk, xc, qzx.v[k]) : 0.0f;
+    d5[k] = u2 ? adj_diff<KAPPA>(sy, -x2, yk, yc, qzy.v[k]) : 0.0f;
+    if (P1) {  // dJ/dcb
+      double g = 0.0;
+      const float c2z = k > 0 ? f1.v[(k + V - 1) % V] : f1z, c0z = k > 0 ? f0.v[(k + V - 1) % V] : f0z;
+      auto term = [&](bool up, float e, float da, float db, float ka, float kb, float pa, float pb) {
+        if (!up) return;
+        const float X = (KAPPA ? ka * da - kb * db : da - db) + (pa - pb);
+        g += (double)e * (double)damp.v[k] * (double)X;
+      };
+      term(u0, a0.v[k], f2.v[k] - f2y.v[k], f1.v[k] - c2z, yk, zk[k], pxy.v[k], pxz[k]);
+      term(u1, a1.v[k], f0.v[k] - c0z, f2.v[k] - f2x.v[k], zk[k], xk, pyz[k], pyx.v[k]);
+      term(u2, a2.v[k], f1.v[k] - f1x.v[k], f0.v[k] - f0y.v[k], xk, yk, pzx.v[k], pzy.v[k]);
+      gc[k] += g;
+    }
+    // psi of the cell: b (psi + u); unchanged where the component is not updated
+    if (XS && u1) qyx.v[k] = xb * (qyx.v[k] - x1);
+    if (XS && u2) qzx.v[k] = xb * (qzx.v[k] + x2);
+    if (YS && u0) qxy.v[k] = yb * (qxy.v[k] + x0);
+    if (YS && u2) qzy.v[k] = yb * (qzy.v[k] - x2);
+    if (ZS && u0) qxz[k] = zb[k] * (qxz[k] - x0);
+    if (ZS && u1) qyz[k] = zb[k] * (qyz[k] + x1);
+  }
+#pragma unroll
+  for (int k = 0; k < V; ++k) {
+    const int z = z0 + k;
+    const bool okz = (CP && !ZS) || (P1 ? z >= 1 : z < nz - 1);
+    const float n0 = ey && okz ? adj_diff<KAPPA>(syn, wy.v[k] * a0y.v[k], ykn, ycn, nxy.v[k]) : 0.0f;
+    const float n5 = ey && okx ? adj_diff<KAPPA>(syn, -(wy.v[k] * a2y.v[k]), ykn, ycn, nzy.v[k]) : 0.0f;
+    const float n3 = ex && okz ? adj_diff<KAPPA>(sxn, -(wx.v[k] * a1x.v[k]), xkn, xcn, nyx.v[k]) : 0.0f;
+    const float n4 = ex && oky ? adj_diff<KAPPA>(sxn, wx.v[k] * a2x.v[k], xkn, xcn, nzx.v[k]) : 0.0f;
+    if (P1) {
+      g0.v[k] = g0.v[k] + (d2[k] - d2[k + 1]) + (d5[k] - n5);
+      g1.v[k] = g1.v[k] + (d1[k] - d1[k + 1]) + (d4[k] - n4);
+      g2.v[k] = g2.v[k] + (d0[k] - n0) + (d3[k] - n3);
+    } else {
+      g0.v[k] = damp.v[k] * g0.v[k] + ((d2[k] - d2[k + 1]) + (n5 - d5[k]));
+      g1.v[k] = damp.v[k] * g1.v[k] + ((d1[k] - d1[k + 1]) + (n4 - d4[k]));
+      g2.v[k] = damp.v[k] * g2.v[k] + ((n0 - d0[k]) + (n3 - d3[k]));
+    }
+  }
+
+  store_v<V>(G[0] + idx, g0);
+  store_v<V>(G[1] + idx, g1);
+  store_v<V>(G[2] + idx, g2);
+  if (P1) {
+    if constexpr (V == 2) *reinterpret_cast<double2*>(p.gcb + idx) = make_double2(gc[0], gc[1]);
+    else p.gcb[idx] = gc[0];
+  }
+  if (XS && sx) {
+    store_v<V>(p.pml.out[QYX] + ox, qyx);
+    store_v<V>(p.pml.out[QZX] + ox, qzx);
+  }
+  if (YS && sy) {
+    store_v<V>(p.pml.out[QXY] + oy, qxy);
+    store_v<V>(p.pml.out[QZY] + oy, qzy);
+  }
+  if (ZS) {
+#pragma unroll
+    for (int k = 0; k < V; ++k)
+      if (sz[k]) {
+        p.pml.out[QXZ][oz + km[k]] = qxz[k];
+        p.pml.out[QYZ][oz + km[k]] = qyz[k];
+      }
   }
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(256) k3a_h(const __grid_constant__ Adj3D p) {
-  const int nx = p.nx, ny = p.ny, nz = p.nz;
-  const long long n = (long long)nx * ny * nz;
-  const long long sx = (long long)ny * nz;
-  constexpr bool CP = (MODE == MODE_CPML);
-  for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < n;
-       j += (long long)gridDim.x * blockDim.x) {
-    int x, y, z;
-    decode_cell(j, nz, ny, p.idx32 != 0, p.div_nz, p.div_ny, x, y, z);
-    // Hbar' = lH + G^T dbarE
-    const float zp_db2 = (z + 1 < nz) ? p.db[2][j + 1] : 0.0f;
-    const float yp_db5 = (y + 1 < ny) ? p.db[5][j + nz] : 0.0f;
-    const float zp_db1 = (z + 1 < nz) ? p.db[1][j + 1] : 0.0f;
-    const float xp_db4 = (x + 1 < nx) ? p.db[4][j + sx] : 0.0f;
-    const float yp_db0 = (y + 1 < ny) ? p.db[0][j + nz] : 0.0f;
-    const float xp_db3 = (x + 1 < nx) ? p.db[3][j + sx] : 0.0f;
-    const float hxb = p.lH[0][j] + (p.db[2][j] - zp_db2) + (p.db[5][j] - yp_db5);
-    const float hyb = p.lH[1][j] + (p.db[1][j] - zp_db1) + (p.db[4][j] - xp_db4);
-    const float hzb = p.lH[2][j] + (p.db[0][j] - yp_db0) + (p.db[3][j] - xp_db3);
-    p.lH[0][j] = hxb;
-    p.lH[1][j] = hyb;
-    p.lH[2][j] = hzb;
-    int im = -1, jm = -1, km = -1;
-    AxisCoef cx{}, cy{}, cz{};
-    if (CP) {
-      im = slab_map(x, nx, p.pml.P[0]);
-      jm = slab_map(y, ny, p.pml.P[1]);
-      km = slab_map(z, nz, p.pml.P[2]);
-      cx = axis_coef(p.pml, 0, x);
-      cy = axis_coef(p.pml, 1, y);
-      cz = axis_coef(p.pml, 2, z);
-    }
-    const long long ix = xs_index(im, y, z, ny, nz);
-    const long long iy = ys_index(x, jm, z, p.pml.L[1], nz);
-    const long long iz = zs_index(x, y, km, ny, p.pml.L[2]);
-    float d[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    auto comp = [&](float hb, bool s1, bool s2, int q1, int q2, long long o1, long long o2,
-                    const AxisCoef& k1, const AxisCoef& k2, int out1, int out2) {
-      const float yb = -p.a * hb;
-      float u1 = yb, u2 = -yb;
-      if (CP && (s1 || s2)) {
-        const float c1 = s1 ? adj_psi(p.lpsi[q1], o1, k1.bh, k1.ch, yb) : 0.0f;
-        const float c2 = s2 ? adj_psi(p.lpsi[q2], o2, k2.bh, k2.ch, -yb) : 0.0f;
-        u1 = k1.ikh * yb + c1;
-        u2 = -k2.ikh * yb + c2;
-      }
-      d[out1] = u1;
-      d[out2] = u2;
-    };
-    if (y < ny - 1 && z < nz - 1)  // Hx: dEz/dy - dEy/dz
-      comp(hxb, jm >= 0, km >= 0, PSI_HXY, PSI_HXZ, iy, iz, cy, cz, 0, 1);
-    if (x < nx - 1 && z < nz - 1)  // Hy: dEx/dz - dEz/dx
-      comp(hyb, km >= 0, im >= 0, PSI_HYZ, PSI_HYX, iz, ix, cz, cx, 2, 3);
-    if (x < nx - 1 && y < ny - 1)  // Hz: dEy/dx - dEx/dy
-      comp(hzb, im >= 0, jm >= 0, PSI_HZX, PSI_HZY, ix, iy, cx, cy, 4, 5);
-    for (int k = 0; k < 6; ++k) p.dh[k][j] = d[k];
-  }
+template <bool P1, int MODE, int V, bool KAPPA, bool CBARR, int REG>
+__device__ __forceinline__ void adj_region(const Adj3D& p, const SweepPlan& s, int x, int b) {
+  constexpr bool YS = REG == 0 || REG == 2, ZS = REG < 2;
+  const int t = b * ADJ_THREADS + (int)threadIdx.x;
+  if (t >= s.r[REG].n) return;
+  const int j = (int)fdiv((uint32_t)t, s.r[REG].dw);
+  const int k = (t - j * s.r[REG].w) * V;
+  const int y = YS ? (j < s.y0 ? j : j + (s.y1 - s.y0)) : s.y0 + j;
+  const int z = ZS ? (k < s.z0 ? k : k + (s.z1 - s.z0)) : s.z0 + k;
+  if (x < s.x0 || x >= s.x1) adj_cells<P1, MODE, V, KAPPA, CBARR, true, YS, ZS>(p, x, y, z);
+  else adj_cells<P1, MODE, V, KAPPA, CBARR, false, YS, ZS>(p, x, y, z);
 }
 
-// Ebar += D^T dbarH (forward differences transposed: gather from i - axis)
-__global__ void __launch_bounds__(256) k3a_e2(const __grid_constant__ Adj3D p) {
-  const int nx = p.nx, ny = p.ny, nz = p.nz;
-  const long long n = (long long)nx * ny * nz;
-  const long long sx = (long long)ny * nz;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    int x, y, z;
-    decode_cell(i, nz, ny, p.idx32 != 0, p.div_nz, p.div_ny, x, y, z);
-    const float zm_dh2 = z >= 1 ? p.dh[2][i - 1] : 0.0f;
-    const float ym_dh5 = y >= 1 ? p.dh[5][i - nz] : 0.0f;
-    const float zm_dh1 = z >= 1 ? p.dh[1][i - 1] : 0.0f;
-    const float xm_dh4 = x >= 1 ? p.dh[4][i - sx] : 0.0f;
-    const float ym_dh0 = y >= 1 ? p.dh[0][i - nz] : 0.0f;
-    const float xm_dh3 = x >= 1 ? p.dh[3][i - sx] : 0.0f;
-    p.lE[0][i] += (zm_dh2 - p.dh[2][i]) + (ym_dh5 - p.dh[5][i]);
-    p.lE[1][i] += (zm_dh1 - p.dh[1][i]) + (xm_dh4 - p.dh[4][i]);
-    p.lE[2][i] += (ym_dh0 - p.dh[0][i]) + (xm_dh3 - p.dh[3][i]);
+// Work split of a plane as in the forward passes (SweepPlan), with one more
+// cell of each slab's inner side in its region: a cell's neighbour is read too.
+template <bool P1, int MODE, int V, bool KAPPA, bool CBARR>
+__global__ void __launch_bounds__(ADJ_THREADS, 5)
+    k3a_pass(const __grid_constant__ Adj3D p, const __grid_constant__ SweepPlan s) {
+  grid_dep_wait();
+  grid_dep_launch_dependents();
+  for (int x = blockIdx.y; x < p.nx; x += gridDim.y) {  // (one plane, below 65,536 of them)
+    int b = blockIdx.x;
+    if (MODE != MODE_CPML) {
+      const int t = b * ADJ_THREADS + (int)threadIdx.x;
+      if (t >= s.r[3].n) return;
+      const int y = (int)fdiv((uint32_t)t, s.r[3].dw);
+      adj_cells<P1, MODE, V, KAPPA, CBARR, false, false, false>(p, x, y, (t - y * s.r[3].w) * V);
+    } else if (b < s.r[0].nb) {
+      adj_region<P1, MODE, V, KAPPA, CBARR, 0>(p, s, x, b);
+    } else if ((b -= s.r[0].nb) < s.r[1].nb) {
+      adj_region<P1, MODE, V, KAPPA, CBARR, 1>(p, s, x, b);
+    } else if ((b -= s.r[1].nb) < s.r[2].nb) {
+      adj_region<P1, MODE, V, KAPPA, CBARR, 2>(p, s, x, b);
+    } else {
+      adj_region<P1, MODE, V, KAPPA, CBARR, 3>(p, s, x, b - s.r[2].nb);
+    }
   }
 }
 
@@ -214,15 +370,17 @@ __global__ void __launch_bounds__(256) k3a_e2(const __grid_constant__ Adj3D p) {
 struct Lam6 {
   float* f[6];  // adjoint of Ex, Ey, Ez, Hx, Hy, Hz
 };
-__global__ void k3a_seed(Lam6 lam, const long long* cell, const int* comp, int n_probes,
+static __global__ void k3a_seed(Lam6 lam, const long long* cell, const int* comp, int n_probes,
                          const float* grad_row) {
+  grid_dep_wait();
+  grid_dep_launch_dependents();
   // one thread: probes may repeat a cell, so add in order
   if (blockIdx.x == 0 && threadIdx.x == 0)
     for (int k = 0; k < n_probes; ++k) lam.f[comp[k]][cell[k]] += grad_row[k];
 }
 
 // dJ/deps_r = dJ/dcb * dcb/deps_r = -dJ/dcb * cb^2 / coef_e
-__global__ void k3a_finish(const double* gcb, const float* cb, float cb_const, double coef_e,
+static __global__ void k3a_finish(const double* gcb, const float* cb, float cb_const, double coef_e,
                            float* grad_eps, long long n) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {

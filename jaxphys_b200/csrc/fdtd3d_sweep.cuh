@@ -68,6 +68,17 @@ struct SweepPlan {
   const SrcTerm* src_term;
 };
 
+// Where an E pass leaves H and the E psi of the step as well (the adjoint's
+// recompute keeps them after every step; a copy would read them again).
+struct SweepSnap {
+  static constexpr bool on = true;
+  float* h[3];
+  float* psi[6];  // EXY .. EZY
+};
+struct NoSnap {
+  static constexpr bool on = false;
+};
+
 template <int V>
 struct VecF {
   float v[V];
@@ -103,8 +114,8 @@ __device__ __forceinline__ void store_v(float* p, const VecF<V>& r) {
 // nor that axis's outer index range can occur, so their code compiles away.
 // Every load is issued before the first store: the psi arrays are updated in
 // place, and a store in between would hold back the loads behind it.
-template <bool H, int MODE, int V, bool KAPPA, bool CBARR, bool XS, bool YS, bool ZS>
-__device__ __forceinline__ void sweep_cells(const Step3D& p, int x, int y, int z0) {
+template <bool H, int MODE, int V, bool KAPPA, bool CBARR, bool XS, bool YS, bool ZS, class SNAP>
+__device__ __forceinline__ void sweep_cells(const Step3D& p, const SNAP& sn, int x, int y, int z0) {
   constexpr bool CP = MODE == MODE_CPML;
   constexpr bool PER = MODE == MODE_PERIODIC;
   constexpr int F = H ? 0 : 3, G = H ? 3 : 0;  // fields read with neighbours / updated
@@ -263,40 +274,50 @@ __device__ __forceinline__ void sweep_cells(const Step3D& p, int x, int y, int z
   store_v<V>(p.out[G] + idx, g0);
   store_v<V>(p.out[G + 1] + idx, g1);
   store_v<V>(p.out[G + 2] + idx, g2);
-  if (XS && xn) {
-    store_v<V>(p.pml.out[Q + PSI_HYX] + ox, qyx);
-    if (yn) store_v<V>(p.pml.out[Q + PSI_HZX] + ox, qzx);
-  }
-  if (YS && yn) {
-    store_v<V>(p.pml.out[Q + PSI_HXY] + oy, qxy);
-    if (xn) store_v<V>(p.pml.out[Q + PSI_HZY] + oy, qzy);
-  }
-  if (ZS) {
+  auto put_psi = [&](float* const* psi) {  // the six arrays of the pass
+    if (XS && xn) {
+      store_v<V>(psi[PSI_HYX] + ox, qyx);
+      if (yn) store_v<V>(psi[PSI_HZX] + ox, qzx);
+    }
+    if (YS && yn) {
+      store_v<V>(psi[PSI_HXY] + oy, qxy);
+      if (xn) store_v<V>(psi[PSI_HZY] + oy, qzy);
+    }
+    if constexpr (ZS) {
 #pragma unroll
-    for (int k = 0; k < V; k += ZP) {
-      float* const u = p.pml.out[Q + PSI_HXZ] + kp[k / ZP];
-      float* const v = p.pml.out[Q + PSI_HYZ] + kp[k / ZP];
-      const int k1 = (k + ZP - 1) % V;
-      if (km[k] >= 0 && km[k1] >= 0) {
-        if (ZP == 2) {
-          if (yn) *reinterpret_cast<float2*>(u) = make_float2(qxz[k], qxz[k1]);
-          if (xn) *reinterpret_cast<float2*>(v) = make_float2(qyz[k], qyz[k1]);
-        } else {
-          if (yn) *u = qxz[k];
-          if (xn) *v = qyz[k];
+      for (int k = 0; k < V; k += ZP) {
+        float* const u = psi[PSI_HXZ] + kp[k / ZP];
+        float* const v = psi[PSI_HYZ] + kp[k / ZP];
+        const int k1 = (k + ZP - 1) % V;
+        if (km[k] >= 0 && km[k1] >= 0) {
+          if (ZP == 2) {
+            if (yn) *reinterpret_cast<float2*>(u) = make_float2(qxz[k], qxz[k1]);
+            if (xn) *reinterpret_cast<float2*>(v) = make_float2(qyz[k], qyz[k1]);
+          } else {
+            if (yn) *u = qxz[k];
+            if (xn) *v = qyz[k];
+          }
+        } else if (ZP == 2 && (km[k] >= 0 || km[k1] >= 0)) {
+          const int i = km[k] >= 0 ? 0 : 1;
+          if (yn) u[i] = i ? qxz[k1] : qxz[k];
+          if (xn) v[i] = i ? qyz[k1] : qyz[k];
         }
-      } else if (ZP == 2 && (km[k] >= 0 || km[k1] >= 0)) {
-        const int i = km[k] >= 0 ? 0 : 1;
-        if (yn) u[i] = i ? qxz[k1] : qxz[k];
-        if (xn) v[i] = i ? qyz[k1] : qyz[k];
       }
     }
+  };
+  if (CP) put_psi(p.pml.out + Q);
+  if constexpr (SNAP::on && !H) {
+    store_v<V>(sn.h[0] + idx, f0);
+    store_v<V>(sn.h[1] + idx, f1);
+    store_v<V>(sn.h[2] + idx, f2);
+    if (CP) put_psi(sn.psi);
   }
 }
 
 // One block of region REG (SweepPlan::r) of plane x.
-template <bool H, int MODE, int V0, int V1, bool KAPPA, bool CBARR, int REG>
-__device__ __forceinline__ void sweep_region(const Step3D& p, const SweepPlan& s, int x, int b) {
+template <bool H, int MODE, int V0, int V1, bool KAPPA, bool CBARR, int REG, class SNAP>
+__device__ __forceinline__ void sweep_region(const Step3D& p, const SweepPlan& s, const SNAP& sn,
+                                             int x, int b) {
   constexpr bool YS = REG == 0 || REG == 2, ZS = REG < 2;
   constexpr int V = ZS ? V1 : V0, NT = sweep_threads(MODE, V0);
   const int t = b * NT + (int)threadIdx.x;
@@ -305,13 +326,14 @@ __device__ __forceinline__ void sweep_region(const Step3D& p, const SweepPlan& s
   const int k = (t - j * s.r[REG].w) * V;
   const int y = YS ? (j < s.y0 ? j : j + (s.y1 - s.y0)) : s.y0 + j;
   const int z = ZS ? (k < s.z0 ? k : k + (s.z1 - s.z0)) : s.z0 + k;
-  if (x < s.x0 || x >= s.x1) sweep_cells<H, MODE, V, KAPPA, CBARR, true, YS, ZS>(p, x, y, z);
-  else sweep_cells<H, MODE, V, KAPPA, CBARR, false, YS, ZS>(p, x, y, z);
+  if (x < s.x0 || x >= s.x1) sweep_cells<H, MODE, V, KAPPA, CBARR, true, YS, ZS>(p, sn, x, y, z);
+  else sweep_cells<H, MODE, V, KAPPA, CBARR, false, YS, ZS>(p, sn, x, y, z);
 }
 
 // Block b of plane x of one grid.
-template <bool H, int MODE, int V0, int V1, bool KAPPA, bool CBARR>
-__device__ __forceinline__ void sweep_block(const Step3D& p, const SweepPlan& s, int x, int b) {
+template <bool H, int MODE, int V0, int V1, bool KAPPA, bool CBARR, class SNAP = NoSnap>
+__device__ __forceinline__ void sweep_block(const Step3D& p, const SweepPlan& s, int x, int b,
+                                            const SNAP& sn = SNAP()) {
   constexpr int NT = sweep_threads(MODE, V0);
   // probes of the state after the previous step: its E components are final
   // until this step's E pass, its H components were recorded by its E pass
@@ -331,16 +353,17 @@ __device__ __forceinline__ void sweep_block(const Step3D& p, const SweepPlan& s,
     const int t = b * NT + (int)threadIdx.x;
     if (t < s.r[3].n) {
       const int y = (int)fdiv((uint32_t)t, s.r[3].dw);
-      sweep_cells<H, MODE, V0, KAPPA, CBARR, false, false, false>(p, x, y, (t - y * s.r[3].w) * V0);
+      sweep_cells<H, MODE, V0, KAPPA, CBARR, false, false, false>(p, sn, x, y,
+                                                                  (t - y * s.r[3].w) * V0);
     }
   } else if (b < s.r[0].nb) {
-    sweep_region<H, MODE, V0, V1, KAPPA, CBARR, 0>(p, s, x, b);
+    sweep_region<H, MODE, V0, V1, KAPPA, CBARR, 0>(p, s, sn, x, b);
   } else if ((b -= s.r[0].nb) < s.r[1].nb) {
-    sweep_region<H, MODE, V0, V1, KAPPA, CBARR, 1>(p, s, x, b);
+    sweep_region<H, MODE, V0, V1, KAPPA, CBARR, 1>(p, s, sn, x, b);
   } else if ((b -= s.r[1].nb) < s.r[2].nb) {
-    sweep_region<H, MODE, V0, V1, KAPPA, CBARR, 2>(p, s, x, b);
+    sweep_region<H, MODE, V0, V1, KAPPA, CBARR, 2>(p, s, sn, x, b);
   } else {
-    sweep_region<H, MODE, V0, V1, KAPPA, CBARR, 3>(p, s, x, b - s.r[2].nb);
+    sweep_region<H, MODE, V0, V1, KAPPA, CBARR, 3>(p, s, sn, x, b - s.r[2].nb);
   }
   // soft sources of the block's cells, after its E update
   if (!H && s0 < s1) {
@@ -364,6 +387,16 @@ __global__ void __launch_bounds__(sweep_threads(MODE, V0), sweep_min_blocks(MODE
   grid_dep_wait();
   grid_dep_launch_dependents();
   sweep_block<H, MODE, V0, V1, KAPPA, CBARR>(p, s, blockIdx.y, blockIdx.x);
+}
+
+// E pass that leaves a snapshot too.
+template <int MODE, int V0, int V1, bool KAPPA, bool CBARR>
+__global__ void __launch_bounds__(sweep_threads(MODE, V0), sweep_min_blocks(MODE, V0))
+    k3d_sweep_snap(const __grid_constant__ Step3D p, const __grid_constant__ SweepPlan s,
+                   const __grid_constant__ SweepSnap sn) {
+  grid_dep_wait();
+  grid_dep_launch_dependents();
+  sweep_block<false, MODE, V0, V1, KAPPA, CBARR, SweepSnap>(p, s, blockIdx.y, blockIdx.x, sn);
 }
 
 // The same pass over several grids of a batch in one launch.  Their parameters

@@ -11,11 +11,14 @@ SweepKernels make(bool cbarr) {
   return SweepKernels{k3d_sweep<true, MODE, V0, V1, KAPPA, false>,
                       cbarr ? k3d_sweep<false, MODE, V0, V1, KAPPA, true>
                             : k3d_sweep<false, MODE, V0, V1, KAPPA, false>,
-                      // (periodic grids are not batched)
+                      // (periodic grids are not batched, and have no adjoint)
                       MODE == MODE_PERIODIC ? nullptr : k3d_sweep_group<true, B, V0, V1, KAPPA, false>,
                       MODE == MODE_PERIODIC ? nullptr
                       : cbarr               ? k3d_sweep_group<false, B, V0, V1, KAPPA, true>
                                             : k3d_sweep_group<false, B, V0, V1, KAPPA, false>,
+                      MODE == MODE_PERIODIC ? nullptr
+                      : cbarr               ? k3d_sweep_snap<B, V0, V1, KAPPA, true>
+                                            : k3d_sweep_snap<B, V0, V1, KAPPA, false>,
                       V0, V1, sweep_threads(MODE, V0)};
 }
 

@@ -8,11 +8,13 @@
 namespace jxf {
 
 using SweepKernel = void (*)(const Step3D, const SweepPlan);
+using SweepSnapKernel = void (*)(const Step3D, const SweepPlan, const SweepSnap);
 using SweepGroupKernel = void (*)(const SweepGroup);
 
 struct SweepKernels {
   SweepKernel h, e;
   SweepGroupKernel group_h, group_e;
+  SweepSnapKernel snap_e;
   int v0, v1;   // cells per thread outside / inside the z slabs
   int threads;  // per block
 };
