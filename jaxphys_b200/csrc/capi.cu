@@ -1325,48 +1325,75 @@ int autotune(jxf_grid3d* g, cudaStream_t st) {
     // fastest), long ones cut the warm-up plane share on large grids
     const int chunks[] = {2, 4, 8, 16, 32, 64};
     const bool can_split = g->mode == MODE_CPML && !g->kappa;
-    for (int sp = 0; sp < 2; ++sp) {
+    // per leapfrog step, trials of about 2 ms or more (small grids run many
+    // steps), best of two
+    const int reps = g->n >= (1LL << 25) ? 3 : (g->n >= (1LL << 21) ? 40 : 100);
+    auto timed = [&](auto&& step, int n, float* ms) -> int {
+      TRY(step());
+      *ms = 1e30f;
+      for (int trial = 0; trial < 2; ++trial) {
+        CUDA_TRY(cudaEventRecord(e0, st));
+        for (int r = 0; r < n; ++r) TRY(step());
+        CUDA_TRY(cudaEventRecord(e1, st));
+        CUDA_TRY(cudaEventSynchronize(e1));
+        float t = 0;
+        CUDA_TRY(cudaEventElapsedTime(&t, e0, e1));
+        *ms = std::min(*ms, t / (float)n);
+      }
+      return JXF_OK;
+    };
+    auto trial_params = [&] {
+      Step3D p = base_params(g);
+      set_io(g, p, g->cur, 1 - g->cur);
+      p.blk_src_ptr = nullptr;
+      p.probe_out = nullptr;
+      p.step = 0;
+      p.err = g->d_err;
+      return p;
+    };
+    auto try_shape = [&](int ci, int ch, int sp) -> int {
+      g->cfg = ci;
+      g->x_chunk = ch;
+      g->axis_split = sp;
+      TRY(encode_maps(g));
+      Step3D p = trial_params();
+      float ms = 0;
+      TRY(timed([&] { return launch_step(g, ci, ch, p, g->cur, st); }, reps, &ms));
+      if (ms < best) {
+        best = ms;
+        bc = ci;
+        bk = ch;
+        bs = sp;
+      }
+      return JXF_OK;
+    };
+    // in-place sweeps, on the idle buffer set
+    float sweep_ms = 1e30f;
+    if (can_sweep && split_env < 0) {
+      TRY(build_sweep(g));
+      Step3D p = base_params(g);
+      TRY(timed([&] { return launch_sweep(g, p, 1 - g->cur, nullptr, false, st); }, reps,
+                &sweep_ms));
+    }
+    // Where they beat the first shape well, the others are not tried: over 64^3
+    // to 224^3 grids of all modes the best launch took 0.58 to 0.99 of the
+    // first shape's time, and trying them all takes 0.5 to 4 s.
+    TRY(try_shape(0, 8, split_env == 1 && can_split ? 1 : 0));
+    const bool sure = sweep_ms < 0.57f * best;
+    for (int sp = 0; sp < 2 && !sure; ++sp) {
       if (sp == 1 && !can_split) continue;
       if (split_env >= 0 && sp != split_env) continue;
-      for (int ci = 0; ci < (int)tma_configs().size(); ++ci) {
+      for (int ci = 0; ci < (int)tma_configs().size(); ++ci)
         for (int ch : chunks) {
           if (ch > g->d.nx && ch != 8) continue;
-          g->cfg = ci;
-          g->x_chunk = ch;
-          g->axis_split = sp;
-          TRY(encode_maps(g));
-          Step3D p = base_params(g);
-          set_io(g, p, g->cur, 1 - g->cur);
-          p.blk_src_ptr = nullptr;
-          p.probe_out = nullptr;
-          p.step = 0;
-          p.err = g->d_err;
-          TRY(launch_step(g, ci, ch, p, g->cur, st));
-          // trials of about 2 ms or more (small grids run many steps), best of two
-          const int reps = g->n >= (1LL << 25) ? 3 : (g->n >= (1LL << 21) ? 40 : 100);
-          float ms = 1e30f;
-          for (int trial = 0; trial < 2; ++trial) {
-            CUDA_TRY(cudaEventRecord(e0, st));
-            for (int r = 0; r < reps; ++r) TRY(launch_step(g, ci, ch, p, g->cur, st));
-            CUDA_TRY(cudaEventRecord(e1, st));
-            CUDA_TRY(cudaEventSynchronize(e1));
-            float t = 0;
-            CUDA_TRY(cudaEventElapsedTime(&t, e0, e1));
-            ms = std::min(ms, t / (float)reps);  // per leapfrog step
-          }
-          if (ms < best) {
-            best = ms;
-            bc = ci;
-            bk = ch;
-            bs = sp;
-          }
+          TRY(try_shape(ci, ch, sp));
         }
-      }
     }
     // two-level blocked launches: time per leapfrog step = launch time / 2
     int btb = -1, btk = 0, bts = bs;
-    if (!tb_off) {
+    if (!tb_off && !sure) {
       const int tchunks[] = {8, 16, 32, 64};
+      const int tb_reps = g->n >= (1LL << 25) ? 2 : (g->n >= (1LL << 21) ? 20 : 50);
       for (int sp = 0; sp < 2; ++sp) {
         if (sp == 1 && !can_split) continue;
         if (split_env >= 0 && sp != split_env) continue;
@@ -1377,25 +1404,11 @@ int autotune(jxf_grid3d* g, cudaStream_t st) {
             g->tb_chunk = ch;
             g->axis_split = sp;
             TRY(encode_maps_tb(g));
-            Step3D p = base_params(g);
-            set_io(g, p, g->cur, 1 - g->cur);
-            p.blk_src_ptr = nullptr;
-            p.probe_out = nullptr;
-            p.step = 0;
-            p.err = g->d_err;
+            Step3D p = trial_params();
             TbExtra ex{};
-            TRY(launch_tb_step(g, ti, ch, p, ex, g->cur, st));
-            const int reps = g->n >= (1LL << 25) ? 2 : (g->n >= (1LL << 21) ? 20 : 50);
-            float ms = 1e30f;
-            for (int trial = 0; trial < 2; ++trial) {
-              CUDA_TRY(cudaEventRecord(e0, st));
-              for (int r = 0; r < reps; ++r) TRY(launch_tb_step(g, ti, ch, p, ex, g->cur, st));
-              CUDA_TRY(cudaEventRecord(e1, st));
-              CUDA_TRY(cudaEventSynchronize(e1));
-              float t = 0;
-              CUDA_TRY(cudaEventElapsedTime(&t, e0, e1));
-              ms = std::min(ms, t / (2.0f * (float)reps));  // two leapfrog steps per launch
-            }
+            float ms = 0;
+            TRY(timed([&] { return launch_tb_step(g, ti, ch, p, ex, g->cur, st); }, tb_reps, &ms));
+            ms *= 0.5f;  // two leapfrog steps per launch
             if (ms < best) {
               best = ms;
               btb = ti;
@@ -1406,26 +1419,7 @@ int autotune(jxf_grid3d* g, cudaStream_t st) {
         }
       }
     }
-    // in-place sweeps, on the idle buffer set
-    if (can_sweep && split_env < 0) {
-      TRY(build_sweep(g));
-      Step3D p = base_params(g);
-      TRY(launch_sweep(g, p, 1 - g->cur, nullptr, false, st));
-      const int reps = g->n >= (1LL << 25) ? 3 : (g->n >= (1LL << 21) ? 40 : 100);
-      for (int trial = 0; trial < 2; ++trial) {
-        CUDA_TRY(cudaEventRecord(e0, st));
-        for (int r = 0; r < reps; ++r)
-          TRY(launch_sweep(g, p, 1 - g->cur, nullptr, false, st));
-        CUDA_TRY(cudaEventRecord(e1, st));
-        CUDA_TRY(cudaEventSynchronize(e1));
-        float t = 0;
-        CUDA_TRY(cudaEventElapsedTime(&t, e0, e1));
-        if (t / (float)reps < best) {
-          best = t / (float)reps;
-          g->sweep = true;
-        }
-      }
-    }
+    g->sweep = sweep_ms < best;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     g->cfg = bc;
