@@ -172,12 +172,14 @@ int jxf_grid3d_run(jxf_grid3d* g, int32_t n_steps, int32_t save_every, int64_t n
  *
  * jxf_grid3d_adjoint_forward: reset, then run n_steps recording the probes
  * into probe_out (device [n_steps][n_probes], may be NULL) and keeping a
- * checkpoint of the full state every checkpoint_every steps (<= 0:
- * ceil(sqrt(n_steps))).
+ * checkpoint of the full state every checkpoint_every steps (<= 0: the H and
+ * psi_E snapshots of as many last steps as fit a sixteenth of the device's
+ * memory and an eighth of what is free are kept, and the steps before them
+ * get checkpoints every ceil(sqrt) of their number).
  * jxf_grid3d_adjoint_backward: probe_grad = dJ/d(probe_out) (device
  * [n_steps][n_probes]); writes dJ/d(eps_r) (device float32 [nx*ny*nz]).
- * Recomputes each segment forward from its checkpoint (one segment of H and
- * psi_E snapshots is held) and runs the adjoint steps in reverse.  Leaves
+ * Recomputes each checkpointed segment forward (one segment of H and psi_E
+ * snapshots is held) and runs the adjoint steps in reverse.  Leaves
  * the grid at its initial (step 0) state.  Not for PERIODIC grids. */
 int jxf_grid3d_adjoint_forward(jxf_grid3d* g, int32_t n_steps, int32_t checkpoint_every,
                                float* probe_out, void* stream);

@@ -302,12 +302,14 @@ struct jxf_grid3d {
   // adjoint (sqrt(T) checkpointing): checkpoints of the full state every
   // adj_k steps, one segment of per-step (H, psiE) snapshots, adjoint state
   int adj_n = 0, adj_k = 0, adj_nseg = 0;
-  size_t adj_state = 0, adj_segstate = 0;  // floats per checkpoint / per snapshot
+  size_t adj_state = 0;     // floats per checkpoint
+  int adj_keep = 0;         // last steps whose snapshots the forward run kept
   float* adj_ck = nullptr;
-  float* adj_sg = nullptr;
+  float* adj_sg = nullptr;  // snapshots of a recomputed segment
+  float* adj_kp = nullptr;  // snapshots of the last adj_keep steps
   float* adj_l = nullptr;   // lE(3n) lH(3n), two sets of lpsi
   double* adj_g = nullptr;  // dJ/dcb
-  size_t adj_ck_cap = 0, adj_sg_cap = 0, adj_l_cap = 0, adj_g_cap = 0;
+  size_t adj_ck_cap = 0, adj_sg_cap = 0, adj_kp_cap = 0, adj_l_cap = 0, adj_g_cap = 0;
   // TMA selection
   int cfg = -1, x_chunk = 0;
   bool maps_ok = false;
@@ -342,6 +344,18 @@ struct jxf_grid3d {
 };
 
 namespace {
+
+size_t psi_size(const jxf_grid3d* g, int id) {
+  static const int axis_of[PSI_COUNT] = {1, 2, 2, 0, 0, 1, 1, 2, 2, 0, 0, 1};
+  const int ax = axis_of[id];
+  if (g->mode != MODE_CPML) return 0;
+  if (ax == 0) return (size_t)g->L[0] * g->d.ny * g->d.nz;
+  if (ax == 1) return (size_t)g->d.nx * g->L[1] * g->d.nz;
+  return (size_t)g->d.nx * g->d.ny * g->L[2];
+}
+
+// arrays of a snapshot start on 16 bytes
+size_t pad4(size_t n) { return (n + 3) / 4 * 4; }
 
 int cells_ok(const jxf_grid3d* g, long long cell) { return cell >= 0 && cell < g->n; }
 
@@ -1693,6 +1707,7 @@ int jxf_grid3d_destroy(jxf_grid3d* g) {
   dfree(g->d_sw_terms);
   dfree(g->adj_ck);
   dfree(g->adj_sg);
+  dfree(g->adj_kp);
   dfree(g->adj_l);
   dfree(g->adj_g);
   dfree(g->d_wave);
@@ -1971,6 +1986,53 @@ static int check_waves3d(const jxf_grid3d* g, long long n_steps) {
   return JXF_OK;
 }
 
+// (a TMA-path grid has been through ensure_tma_ready)
+static bool steps_by_sweep(const jxf_grid3d* g) {
+  return g->sweep || (g->path == JXF_PATH_GENERIC && sweep_ok(g));
+}
+
+// Floats of a snapshot (H and the E psi after a step), and one at `base`.
+static size_t snap_floats(const jxf_grid3d* g) {
+  size_t n = 3 * pad4((size_t)g->n);
+  for (int k = PSI_EXY; k < PSI_COUNT; ++k) n += pad4(psi_size(g, k));
+  return n;
+}
+static SweepSnap snap_at(const jxf_grid3d* g, float* base) {
+  SweepSnap sn{};
+  for (int c = 0; c < 3; ++c) {
+    sn.h[c] = base;
+    base += pad4((size_t)g->n);
+  }
+  for (int q = 0; q < 6; ++q) {
+    sn.psi[q] = base;
+    base += pad4(psi_size(g, PSI_EXY + q));
+  }
+  return sn;
+}
+
+// n steps on the in-place passes; snaps: snapshots of consecutive steps, or
+// null (not with a learned band).
+static int sweep_steps(jxf_grid3d* g, Step3D& p, int n, float* probe_out, cudaStream_t st,
+                       float* snaps) {
+  TRY(build_sweep(g));
+  const int np = g->n_probes;
+  const bool record = probe_out && np > 0;
+  const bool fused = record && sweep_records(g, g->band.band != nullptr);
+  for (int k = 0; k < n; ++k) {
+    float* const row = record ? probe_out + (size_t)k * np : nullptr;
+    SweepSnap sn;
+    if (snaps) sn = snap_at(g, snaps + (size_t)k * snap_floats(g));
+    p.step = g->step;
+    p.probe_out = fused && k > 0 ? row - np : nullptr;
+    TRY(launch_sweep(g, p, g->cur, fused ? row : nullptr, !g->src_cell.empty(), st,
+                     snaps ? &sn : nullptr));
+    g->step++;
+    if (g->band.band) TRY(band_launch(g->band, st, g->cur, g->use_pdl));
+    if (record && (!fused || k + 1 == n)) TRY(gather_probes(g, g->cur, row, st));
+  }
+  return JXF_OK;
+}
+
 int jxf_grid3d_step(jxf_grid3d* g, int32_t n_steps, float* probe_out, void* stream) {
   if (!g) return fail(JXF_ERR_INVALID, "null handle");
   if (g->slab && g->path != JXF_PATH_TMA)
@@ -1987,19 +2049,8 @@ int jxf_grid3d_step(jxf_grid3d* g, int32_t n_steps, float* probe_out, void* stre
   Step3D p = base_params(g);
   const int np = g->n_probes;
   if (g->path == JXF_PATH_TMA) TRY(ensure_tma_ready(g, st));
-  if (g->sweep || (g->path == JXF_PATH_GENERIC && sweep_ok(g))) {
-    TRY(build_sweep(g));
-    const bool record = probe_out && np > 0;
-    const bool fused = record && sweep_records(g, g->band.band != nullptr);
-    for (int k = 0; k < n_steps; ++k) {
-      float* const row = record ? probe_out + (size_t)k * np : nullptr;
-      p.step = g->step;
-      p.probe_out = fused && k > 0 ? row - np : nullptr;
-      TRY(launch_sweep(g, p, g->cur, fused ? row : nullptr, !g->src_cell.empty(), st));
-      g->step++;
-      if (g->band.band) TRY(band_launch(g->band, st, g->cur, g->use_pdl));
-      if (record && (!fused || k + 1 == n_steps)) TRY(gather_probes(g, g->cur, row, st));
-    }
+  if (steps_by_sweep(g)) {
+    TRY(sweep_steps(g, p, n_steps, probe_out, st, nullptr));
   } else if (g->path == JXF_PATH_TMA) {
     p.blk_src_ptr = g->src_cell.empty() ? nullptr : g->d_blk_ptr;
     p.src = g->d_entries;
@@ -4399,18 +4450,6 @@ int jxf_grid3d_set_band(jxf_grid3d* g, jxf_band* m) {
 
 namespace {
 
-size_t psi_size(const jxf_grid3d* g, int id) {
-  static const int axis_of[PSI_COUNT] = {1, 2, 2, 0, 0, 1, 1, 2, 2, 0, 0, 1};
-  const int ax = axis_of[id];
-  if (g->mode != MODE_CPML) return 0;
-  if (ax == 0) return (size_t)g->L[0] * g->d.ny * g->d.nz;
-  if (ax == 1) return (size_t)g->d.nx * g->L[1] * g->d.nz;
-  return (size_t)g->d.nx * g->d.ny * g->L[2];
-}
-
-// arrays of a snapshot start on 16 bytes
-size_t pad4(size_t n) { return (n + 3) / 4 * 4; }
-
 template <class T>
 int ensure_buf(T** p, size_t* cap, size_t count, int64_t* tally) {
   if (*cap >= count && *p) return JXF_OK;
@@ -4496,25 +4535,54 @@ extern "C" int jxf_grid3d_adjoint_forward(jxf_grid3d* g, int32_t n_steps,
     return fail(JXF_ERR_INVALID, "the adjoint supports ABSORBING, PEC and CPML boundaries");
   DeviceGuard dg(g->d.device);
   cudaStream_t st = (cudaStream_t)stream;
-  const int K = checkpoint_every > 0 ? checkpoint_every
-                                     : std::max(1, (int)std::ceil(std::sqrt((double)n_steps)));
-  const int nseg = (n_steps + K - 1) / K;
-  size_t state = 6 * (size_t)g->n, segstate = 3 * pad4((size_t)g->n);
+  const size_t snap = snap_floats(g);
+  size_t state = 6 * (size_t)g->n;
   for (int k = 0; k < PSI_COUNT; ++k) state += psi_size(g, k);
-  for (int k = PSI_EXY; k < PSI_COUNT; ++k) segstate += pad4(psi_size(g, k));
-  TRY(ensure_buf(&g->adj_ck, &g->adj_ck_cap, state * nseg, &g->bytes));
+  if (g->path == JXF_PATH_TMA) TRY(ensure_tma_ready(g, st));
+  // Where the caller leaves the memory to the library, the snapshots of as
+  // many last steps as fit a sixteenth of the device (and an eighth of what is
+  // free of it) are kept, and only the steps before them are recomputed: a
+  // recomputed step costs as much as a forward one (96^3, 2000 steps, 650 of
+  // them kept in 11 GB: 104.8 ms a gradient against 116.7; 48^3, 300 steps, all
+  // kept: 5.96 against 8.60).
+  // JXF_ADJ_KEEP=steps caps it.
+  int keep = 0;
+  const char* env = std::getenv("JXF_ADJ_KEEP");
+  const int most = env ? std::max(0, std::min(n_steps, std::atoi(env))) : n_steps;
+  if (checkpoint_every <= 0 && most > 0 && steps_by_sweep(g) && !g->band.band) {
+    const size_t want = snap * (size_t)most;
+    if (g->adj_kp_cap < want) {
+      size_t free_b = 0, total_b = 0;
+      CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
+      const size_t may = std::min(total_b / 16, (free_b + 4 * g->adj_kp_cap) / 8) / 4;
+      if (may > g->adj_kp_cap &&
+          ensure_buf(&g->adj_kp, &g->adj_kp_cap, std::min(want, may / snap * snap), &g->bytes) != JXF_OK)
+        (void)cudaGetLastError();  // no room: recompute
+    }
+    keep = (int)std::min<size_t>(most, g->adj_kp_cap / snap);
+  }
+  const int m = n_steps - keep;  // steps from checkpoints
+  const int K = checkpoint_every > 0 ? checkpoint_every
+                                     : std::max(1, (int)std::ceil(std::sqrt((double)m)));
+  const int nseg = (m + K - 1) / K;
+  if (nseg > 0) TRY(ensure_buf(&g->adj_ck, &g->adj_ck_cap, state * nseg, &g->bytes));
   TRY(jxf_grid3d_reset(g, stream));
+  TRY(check_waves3d(g, n_steps));
   const int np = g->n_probes;
   for (int s = 0; s < nseg; ++s) {
-    const int start = s * K, len = std::min(K, n_steps - start);
+    const int start = s * K, len = std::min(K, m - start);
     TRY(ckpt_copy(g, g->adj_ck + (size_t)s * state, true, st));
     TRY(jxf_grid3d_step(g, len, probe_out ? probe_out + (size_t)start * np : nullptr, stream));
+  }
+  if (keep > 0) {
+    Step3D p = base_params(g);
+    TRY(sweep_steps(g, p, keep, probe_out ? probe_out + (size_t)m * np : nullptr, st, g->adj_kp));
   }
   g->adj_n = n_steps;
   g->adj_k = K;
   g->adj_nseg = nseg;
   g->adj_state = state;
-  g->adj_segstate = segstate;
+  g->adj_keep = keep;
   return JXF_OK;
 }
 
@@ -4529,7 +4597,8 @@ extern "C" int jxf_grid3d_adjoint_backward(jxf_grid3d* g, const float* probe_gra
   const int K = g->adj_k, N = g->adj_n;
   size_t psi_tot = 0;
   for (int k = 0; k < PSI_COUNT; ++k) psi_tot += psi_size(g, k);
-  TRY(ensure_buf(&g->adj_sg, &g->adj_sg_cap, g->adj_segstate * K, &g->bytes));
+  const size_t snap = snap_floats(g);
+  if (g->adj_nseg > 0) TRY(ensure_buf(&g->adj_sg, &g->adj_sg_cap, snap * K, &g->bytes));
   // adjoint fields, and two sets of adjoint psi
   TRY(ensure_buf(&g->adj_l, &g->adj_l_cap, 6 * n + 2 * psi_tot, &g->bytes));
   TRY(ensure_buf(&g->adj_g, &g->adj_g_cap, n, &g->bytes));
@@ -4577,83 +4646,60 @@ extern "C" int jxf_grid3d_adjoint_backward(jxf_grid3d* g, const float* probe_gra
   lc.stream = st;
   lc.attrs = attr;
   lc.numAttrs = g->use_pdl ? 1 : 0;
+  int set = 0;  // adjoint psi before the step
+  auto adjoint_step = [&](int step_n, float* snapshot) -> int {
+    if (np > 0) {
+      lc.gridDim = dim3(1, 1, 1);
+      lc.blockDim = dim3(32, 1, 1);
+      CUDA_TRY(cudaLaunchKernelEx(&lc, k3a_seed, lam, (const long long*)g->d_probe_cell,
+                                  (const int*)g->d_probe_comp, np,
+                                  probe_grad + (size_t)step_n * np));
+    }
+    const SweepSnap sn = snap_at(g, snapshot);
+    for (int c = 0; c < 3; ++c) a.fh[c] = sn.h[c];
+    for (int q = 0; q < 6; ++q) a.fpsiE[q] = sn.psi[q];
+    for (int q = 0; q < PSI_COUNT; ++q) {
+      a.pml.in[q] = lpsi[set][q];
+      a.pml.out[q] = lpsi[set ^ 1][q];
+    }
+    set ^= 1;
+    lc.gridDim = dim3(plan.nblk, std::min(g->d.nx, 65535), 1);
+    lc.blockDim = dim3(ADJ_THREADS, 1, 1);
+    CUDA_TRY(cudaLaunchKernelEx(&lc, ak.e, a, plan));
+    CUDA_TRY(cudaLaunchKernelEx(&lc, ak.h, a, plan));
+    return JXF_OK;
+  };
+  const int m = N - g->adj_keep;
+  for (int k = g->adj_keep - 1; k >= 0; --k)
+    TRY(adjoint_step(m + k, g->adj_kp + (size_t)k * snap));
   // segments recomputed on the in-place passes leave their snapshots from the
   // E pass; other launches (and a band, which corrects the state) are copied
   if (g->path == JXF_PATH_TMA) TRY(ensure_tma_ready(g, st));
-  const bool in_pass =
-      (g->sweep || (g->path == JXF_PATH_GENERIC && sweep_ok(g))) && !g->band.band;
-  if (in_pass) TRY(build_sweep(g));
+  const bool in_pass = steps_by_sweep(g) && !g->band.band;
   Step3D sp = base_params(g);
-
-  int set = 0;  // adjoint psi before the step
   for (int s = g->adj_nseg - 1; s >= 0; --s) {
-    const int start = s * K, len = std::min(K, N - start);
+    const int start = s * K, len = std::min(K, m - start);
     // recompute the segment, keeping (H, psiE) after every step
     TRY(ckpt_copy(g, g->adj_ck + (size_t)s * g->adj_state, false, st));
     g->step = start;
     TRY(check_waves3d(g, len));
-    for (int k = 0; k < len; ++k) {
-      SweepSnap sn{};
-      size_t off = (size_t)k * g->adj_segstate;
-      for (int c = 0; c < 3; ++c) {
-        sn.h[c] = g->adj_sg + off;
-        off += pad4(n);
-      }
-      for (int q = 0; q < 6; ++q) {
-        sn.psi[q] = g->adj_sg + off;
-        off += pad4(psi_size(g, PSI_EXY + q));
-      }
-      if (in_pass) {
-        sp.step = g->step;
-        sp.probe_out = nullptr;
-        TRY(launch_sweep(g, sp, g->cur, nullptr, !g->src_cell.empty(), st, &sn));
-        g->step++;
-        continue;
-      }
+    if (in_pass) TRY(sweep_steps(g, sp, len, nullptr, st, g->adj_sg));
+    for (int k = 0; k < len && !in_pass; ++k) {
       TRY(jxf_grid3d_step(g, 1, nullptr, stream));
+      const SweepSnap sn = snap_at(g, g->adj_sg + (size_t)k * snap);
       CopyBatch cb;
       for (int c = 0; c < 3; ++c) cb.add(sn.h[c], g->f[g->cur][3 + c], n);
       for (int q = 0; q < 6; ++q)
         cb.add(sn.psi[q], g->psi[g->cur][PSI_EXY + q], psi_size(g, PSI_EXY + q));
       TRY(cb.launch(st));
     }
-    // adjoint steps, last to first
-    for (int k = len - 1; k >= 0; --k) {
-      const int step_n = start + k;
-      if (np > 0) {
-        lc.gridDim = dim3(1, 1, 1);
-        lc.blockDim = dim3(32, 1, 1);
-        CUDA_TRY(cudaLaunchKernelEx(&lc, k3a_seed, lam, (const long long*)g->d_probe_cell,
-                                    (const int*)g->d_probe_comp, np,
-                                    probe_grad + (size_t)step_n * np));
-      }
-      size_t off = (size_t)k * g->adj_segstate;
-      for (int c = 0; c < 3; ++c) {
-        a.fh[c] = g->adj_sg + off;
-        off += pad4(n);
-      }
-      for (int q = 0; q < 6; ++q) {
-        a.fpsiE[q] = g->adj_sg + off;
-        off += pad4(psi_size(g, PSI_EXY + q));
-      }
-      for (int q = 0; q < PSI_COUNT; ++q) {
-        a.pml.in[q] = lpsi[set][q];
-        a.pml.out[q] = lpsi[set ^ 1][q];
-      }
-      set ^= 1;
-      lc.gridDim = dim3(plan.nblk, std::min(g->d.nx, 65535), 1);
-      lc.blockDim = dim3(ADJ_THREADS, 1, 1);
-      CUDA_TRY(cudaLaunchKernelEx(&lc, ak.e, a, plan));
-      CUDA_TRY(cudaLaunchKernelEx(&lc, ak.h, a, plan));
-    }
+    for (int k = len - 1; k >= 0; --k)
+      TRY(adjoint_step(start + k, g->adj_sg + (size_t)k * snap));
   }
   k3a_finish<<<blocks, threads, 0, st>>>(g->adj_g, g->cb, (float)g->coef_e, g->coef_e, grad_eps,
                                          (long long)n);
   CUDA_TRY(cudaGetLastError());
-  // leave the grid at its initial state
-  TRY(ckpt_copy(g, g->adj_ck, false, st));
-  g->step = 0;
-  return JXF_OK;
+  return jxf_grid3d_reset(g, stream);  // leave the grid at its initial state
 }
 
 // ---------------------------------------------------------------------------

@@ -477,8 +477,11 @@ class EMGrid3D:
 
     # ------------------------------------------------------------- adjoint
     def adjoint_forward(self, n_steps: int, checkpoint_every: int | None = None):
-        """Extension: reset, run ``n_steps`` keeping sqrt(T) checkpoints for
-        :meth:`adjoint_backward`; returns the probe traces (n_steps, P)."""
+        """Extension: reset, run ``n_steps`` keeping what
+        :meth:`adjoint_backward` needs: a checkpoint every ``checkpoint_every``
+        steps, or by default the snapshots of as many last steps as fit a
+        sixteenth of the device and sqrt(T) checkpoints of the others; returns
+        the probe traces (n_steps, P)."""
         import torch
 
         if self._h is None:

@@ -20,7 +20,7 @@ pytestmark = pytest.mark.gpu
 STEPS = 60
 
 
-def _compare(cuda, size, layers, boundary, path, sources, probes):
+def _compare(cuda, size, layers, boundary, path, sources, probes, every=9):
     import torch
 
     from jaxphys_b200 import CPMLSpec, EMGrid3D, PointSource3D
@@ -47,7 +47,7 @@ def _compare(cuda, size, layers, boundary, path, sources, probes):
     w = np.random.default_rng(1).random((STEPS, len(probes)))
     w[:, 3:] *= 377.0**2
     e = torch.tensor(eps, dtype=torch.float32, device=cuda, requires_grad=True)
-    tr = probe_traces(g, e, STEPS, checkpoint_every=9)
+    tr = probe_traces(g, e, STEPS, checkpoint_every=every)
     (torch.as_tensor(w, dtype=torch.float32, device=cuda) * tr**2).sum().backward()
 
     src64 = [dict(position=s["position"], polarization=s["polarization"],
@@ -90,3 +90,15 @@ def test_gradient_in_damping_layers(cuda, size):
     probes = [(*c, 0), (c[0] - 1, c[1], c[2] + 2, 2), (c[0] + 1, c[1] - 2, c[2], 4)]
     sources = [(0.06, c, "z", 5.0, 1.0), (0.05, (c[0], c[1] + 2, c[2] - 2), "x", 4.0, 0.7)]
     _compare(cuda, size, 3, "absorbing", "auto", sources, probes)
+
+
+@pytest.mark.parametrize("keep", [None, "0", "25", "59"])
+def test_kept_and_recomputed_steps(cuda, monkeypatch, keep):
+    """Snapshots kept by the forward run for all, none, some and all but one
+    of the steps."""
+    if keep is not None:
+        monkeypatch.setenv("JXF_ADJ_KEEP", keep)
+    size = (12, 15, 14)
+    sources = [(0.06, (6, 7, 7), "z", 5.0, 1.0), (0.05, (1, 13, 1), "x", 4.0, 0.7)]
+    probes = [(6, 7, 12, 2), (11, 2, 2, 1), (2, 0, 7, 3)]
+    _compare(cuda, size, 3, "cpml", "auto", sources, probes, every=None)
