@@ -355,7 +355,9 @@ def run_ours(args, world, rank, local, pg, workload=None, steps=None, warmup=Non
                      "peak_source": peak_kind, "bytes_per_cell_update": round(b_cell, 2),
                      "kernel": ("k3d_tb2 two-level blocked pass (every launch of a pass), "
                                 "per leapfrog step" if blocked else
-                                "k3d_tma step (every launch of one leapfrog step)"),
+                                "k3d_tma step (every launch of one leapfrog step)"
+                                if launch["tma_config"] >= 0 else
+                                "k3d_sweep H and E passes (two launches of one leapfrog step)"),
                      "ms_per_leapfrog_step": round(per_launch_ms, 5)},
         "gpu_launches": launches * n_timed,
         "clocks": clocks,
@@ -443,13 +445,13 @@ def run_batch(args, world, rank, local, pg, steps=None, warmup=None, reflection=
     def build(kind):
         grids = []
         for c in cases:
-            # every c5 grid is padded to nz % 4 == 0: the batch runs on the
-            # persistent TMA kernel
+            # every c5 grid is padded to nz % 4 == 0: the batch chooses between
+            # the persistent TMA kernel and in-place passes
             if kind in ("learned", "pec"):
-                g = c.grid(BAND_LAYERS, "pec", 0, path="tma")
+                g = c.grid(BAND_LAYERS, "pec", 0, path="auto")
             else:
                 k = int(kind[4:])
-                g = c.grid(k, "cpml", k, path="tma")
+                g = c.grid(k, "cpml", k, path="auto")
             g.prepare()
             grids.append(g)
         b = FDTDBatch(grids)
@@ -535,7 +537,10 @@ def run_batch(args, world, rank, local, pg, steps=None, warmup=None, reflection=
         "config": {"workload": wname, "grids": n_grids, "interior_cells": interior_total,
                    "leapfrog_steps_per_step": nsteps, "band_layers": BAND_LAYERS,
                    "l2": "inputs larger than L2 (>= 360 MB of fields)",
-                   "path": "tma (persistent batch launch)", "launch": lr.pop("launch", None),
+                   "path": ("tma (persistent batch launch)"
+                            if lr.get("launch", {}).get("tma_config", -1) >= 0
+                            else "in-place passes, group by group"),
+                   "launch": lr.pop("launch", None),
                    "parallelism": f"the {n_grids} grids bin-packed by cell count over {world} GPU(s)"},
         "compare": {k: results[k] for k in ("cpml10", "cpml4", "pec") if k in results},
         "reflection_db": refl,
