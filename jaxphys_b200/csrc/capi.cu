@@ -2504,7 +2504,7 @@ Block2DConfig make_block2d(double launch, double lat0, double lat1, double thr0,
 }
 const std::vector<Block2DConfig>& block2d_configs() {
   static const std::vector<Block2DConfig> c = {
-      make_block2d<32, 16, 2>(3.4, 0.48, 0.70, 0.21, 0.23),
+      make_block2d<32, 16, 2>(3.4, 0.48, 0.66, 0.21, 0.27),
       make_block2d<64, 16, 4>(5.6, 0.82, 1.28, 0.62, 0.72)};
   return c;
 }
