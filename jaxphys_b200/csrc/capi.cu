@@ -310,6 +310,7 @@ struct jxf_grid3d {
   float* adj_l = nullptr;   // lE(3n) lH(3n), two sets of lpsi
   double* adj_g = nullptr;  // dJ/dcb
   size_t adj_ck_cap = 0, adj_sg_cap = 0, adj_kp_cap = 0, adj_l_cap = 0, adj_g_cap = 0;
+  size_t adj_kp_want = 0;  // floats that adj_kp was last sized for
   // TMA selection
   int cfg = -1, x_chunk = 0;
   bool maps_ok = false;
@@ -4545,19 +4546,30 @@ extern "C" int jxf_grid3d_adjoint_forward(jxf_grid3d* g, int32_t n_steps,
   // recomputed step costs as much as a forward one (96^3, 2000 steps, 650 of
   // them kept in 11 GB: 104.8 ms a gradient against 116.7; 48^3, 300 steps, all
   // kept: 5.96 against 8.60).
+  // The eighth is of what is left beside everything else that this call and
+  // the backward one allocate, so a gradient that fits without it still fits;
+  // and the buffer is sized once for a step count, so that repeated calls (a
+  // captured one among them) neither allocate nor ask for the free memory.
   // JXF_ADJ_KEEP=steps caps it.
   int keep = 0;
   const char* env = std::getenv("JXF_ADJ_KEEP");
   const int most = env ? std::max(0, std::min(n_steps, std::atoi(env))) : n_steps;
   if (checkpoint_every <= 0 && most > 0 && steps_by_sweep(g) && !g->band.band) {
     const size_t want = snap * (size_t)most;
-    if (g->adj_kp_cap < want) {
+    if (g->adj_kp_want < want) {
       size_t free_b = 0, total_b = 0;
       CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-      const size_t may = std::min(total_b / 16, (free_b + 4 * g->adj_kp_cap) / 8) / 4;
-      if (may > g->adj_kp_cap &&
-          ensure_buf(&g->adj_kp, &g->adj_kp_cap, std::min(want, may / snap * snap), &g->bytes) != JXF_OK)
+      free_b += 4 * g->adj_kp_cap;
+      const size_t kk = (size_t)std::ceil(std::sqrt((double)n_steps));
+      // checkpoints, a segment's snapshots, adjoint fields and two psi sets,
+      // dJ/dcb in FP64
+      const size_t rest = 4 * ((kk + 1) * state + kk * snap + 2 * state);
+      const size_t may = std::min(total_b / 16, (free_b > rest ? free_b - rest : 0) / 8) / 4;
+      const size_t get = std::min(want, may / snap * snap);
+      if (get > g->adj_kp_cap &&
+          ensure_buf(&g->adj_kp, &g->adj_kp_cap, get, &g->bytes) != JXF_OK)
         (void)cudaGetLastError();  // no room: recompute
+      g->adj_kp_want = want;
     }
     keep = (int)std::min<size_t>(most, g->adj_kp_cap / snap);
   }

@@ -102,3 +102,33 @@ def test_kept_and_recomputed_steps(cuda, monkeypatch, keep):
     sources = [(0.06, (6, 7, 7), "z", 5.0, 1.0), (0.05, (1, 13, 1), "x", 4.0, 0.7)]
     probes = [(6, 7, 12, 2), (11, 2, 2, 1), (2, 0, 7, 3)]
     _compare(cuda, size, 3, "cpml", "auto", sources, probes, every=None)
+
+
+def test_step_counts_in_turn(cuda):
+    """The buffer of kept snapshots is sized for the longest run so far: runs
+    of other lengths on the same grid give what a new grid gives."""
+    import torch
+
+    from jaxphys_b200 import EMGrid3D, PointSource3D
+    from jaxphys_b200.em.adjoint import probe_traces
+
+    size = (12, 15, 14)
+    eps = torch.tensor(smooth_eps(size, 1.0, 4.0, seed=7), dtype=torch.float32, device=cuda)
+
+    def grid():
+        g = EMGrid3D(size=size, resolution=1.0, boundary="cpml", pml_layers=3)
+        g.add_source(PointSource3D(frequency=0.06 / rn.default_dt_3d(1.0), position=(6, 7, 7),
+                                   waveform="gauss_sine", width_steps=5.0))
+        g.add_probe((6, 7, 12), "ez")
+        g.prepare(dt=rn.default_dt_3d(1.0))
+        return g
+
+    def grad(g, steps):
+        e = eps.clone().requires_grad_(True)
+        (probe_traces(g, e, steps) ** 2).sum().backward()
+        return to_np(e.grad)
+
+    used = grid()
+    for steps in (30, 60, 1, 45, 60):
+        got = grad(used, steps)
+        assert np.array_equal(got, grad(grid(), steps)), steps
