@@ -343,7 +343,8 @@ def run_ours(args, world, rank, local, pg, workload=None, steps=None, warmup=Non
         "data": "synthetic (seeded eps_r sphere, pulsed dipole, seeded probes)",
         "config": {"workload": wname, "cells": cells, "leapfrog_steps_per_step": nsteps,
                    "boundary": "cpml", "pml_layers": pml, "l2": "flushed (256 MiB write) between steps",
-                   "path": "tma" if info["path"] == 2 else "generic",
+                   "path": ("generic" if info["path"] != 2 else
+                            "tma" if info["tma_config"] >= 0 else "in-place passes"),
                    "tile": [info["tile_z"], info["tile_y"], info["rows_per_thread"],
                             info["stages"], info["x_chunk"]],
                    "launch": launch,

@@ -13,12 +13,14 @@
 // 126 MB L2 from step to step, while the marching kernel's two sets do not
 // fit, and its march is a serial chain of planes with a barrier in each.  Here
 // every load of a thread is in flight at once and there is no barrier.  What
-// bounds the passes is L2 to SM traffic (the 128^3 CPML passes move 66 and 73
-// bytes per cell at 12 TB/s), below 64^3 the two launches of a step (about
-// 2.4 us each).  Measured per step on one B200, against the kernels used
-// before: 128^3 10-layer CPML 24.7 us (marching kernel 41.1), 64^3 8-layer
-// CPML 8.1 us (10.5), 60^3 absorbing 5.0 us (11), 96 x 80 x 64 periodic 6.5 us
-// (per-cell kernels, three launches: 18), 75 x 90 x 61 CPML 11.8 us (24).
+// bounds the passes is the L1 of each SM (0.65 busy in a profiled 128^3 CPML
+// pass of 17.7 us that takes 12.2 unprofiled) and the wait for its loads, at
+// 66 and 73 bytes per cell, 12 TB/s, in the two passes; below 64^3 the two
+// launches of a step (about 2.4 us each).  Measured per step on one B200,
+// against the kernels used before: 128^3 10-layer CPML 24.7 us (marching
+// kernel 41.1), 64^3 8-layer CPML 8.1 us (10.5), 60^3 absorbing 5.0 us (11),
+// 96 x 80 x 64 periodic 6.5 us (per-cell kernels, three launches: 18),
+// 75 x 90 x 61 CPML 11.8 us (24).
 // Above L2 size it is bound by DRAM (76 bytes per cell and step against 52),
 // and the autotuner takes the marching or the blocked kernel there.
 #pragma once
@@ -143,6 +145,7 @@ __device__ __forceinline__ void sweep_cells(const Step3D& p, const SNAP& sn, int
   const VecF<V> f2 = load_v<V>(p.in[F + 2] + idx);
   const VecF<V> f0y = load_v<V>(p.in[F] + iy), f2y = load_v<V>(p.in[F + 2] + iy);
   const VecF<V> f1x = load_v<V>(p.in[F + 1] + ix), f2x = load_v<V>(p.in[F + 2] + ix);
+  // (from the next lane by a shuffle instead: 128^3 CPML 26.6 us a step, not 24.3)
   const float f0z = p.in[F][iz], f1z = p.in[F + 1][iz];
   VecF<V> g0 = load_v<V>(p.in[G] + idx);
   VecF<V> g1 = load_v<V>(p.in[G + 1] + idx);

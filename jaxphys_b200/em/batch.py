@@ -4,6 +4,9 @@
 boundary mode, all on one kernel path, and advances all of them together (C
 ABI ``jxf_batch3d_*``):
 
+* in-place passes (every grid ``path="auto"``; chosen on the first run where
+  they are faster): groups of grids that stay in the L2 cache, each running
+  all its steps before the next group begins.
 * TMA path (nz % 4 == 0; ``path="auto"`` or ``"tma"``): one persistent launch
   per step (and per CPML part) over a work list of every grid's
   (tile, x-chunk) blocks, heaviest first; blocks take work through an atomic
@@ -13,8 +16,8 @@ ABI ``jxf_batch3d_*``):
 * generic path: one kernel per phase per step over the whole batch (any
   shape, odd nz included).
 
-``run(n)`` captures the n-step sequence once into a CUDA graph and replays it
-with a single launch.  Each grid keeps its own permittivity, sources, probes
+``run(n)`` of the last two captures the n-step sequence once into a CUDA graph
+and replays it with a single launch.  Each grid keeps its own permittivity, sources, probes
 and field accessors.  Typical use: many design candidates, or many source
 positions, of one device.
 """
