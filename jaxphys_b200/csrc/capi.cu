@@ -83,9 +83,18 @@ struct DeviceGuard {
 };
 
 // Fault injection for the failure-detection tests: JXF_FAULT_ALLOC_AFTER=n
-// (read when a grid is created) lets the next n device allocations of that
-// creation succeed and fails the one after with JXF_ERR_OOM.
+// (read when a grid is created and when a batch steps) lets the next n device
+// allocations of that call succeed and fails the one after with JXF_ERR_OOM.
 thread_local long long g_alloc_budget = -1;
+
+// JXF_FAULT_ALLOC_AFTER for the length of one call.
+struct AllocFault {
+  AllocFault() {
+    const char* e = std::getenv("JXF_FAULT_ALLOC_AFTER");
+    g_alloc_budget = (e && *e) ? std::max(0LL, std::atoll(e)) : -1;
+  }
+  ~AllocFault() { g_alloc_budget = -1; }
+};
 
 template <class T>
 int dmalloc(T** p, size_t count, int64_t* tally) {
@@ -1536,11 +1545,8 @@ static int create3d_impl(const jxf_grid3d_desc& d, int gnx, int gx0, int x_lo, i
 
 static int create3d(const jxf_grid3d_desc& d, int gnx, int gx0, int x_lo, int x_hi, bool slab,
                     jxf_grid3d** out) {
-  const char* e = std::getenv("JXF_FAULT_ALLOC_AFTER");
-  g_alloc_budget = (e && *e) ? std::max(0LL, std::atoll(e)) : -1;
-  const int rc = create3d_impl(d, gnx, gx0, x_lo, x_hi, slab, out);
-  g_alloc_budget = -1;
-  return rc;
+  const AllocFault fault;
+  return create3d_impl(d, gnx, gx0, x_lo, x_hi, slab, out);
 }
 
 static int create3d_impl(const jxf_grid3d_desc& d, int gnx, int gx0, int x_lo, int x_hi,
@@ -3347,8 +3353,10 @@ int batch_sweep_groups(jxf_batch3d* b) {
   };
   // (a permittivity map set or dropped since changes a grid's kernel)
   bool current = !b->groups.empty();
-  for (const auto& gr : b->groups)
+  for (const auto& gr : b->groups) {
+    current = current && gr.band.band == b->band.band;
     for (int k : gr.grids) current = current && kernel_of(k) == kernel_of(gr.grids[0]);
+  }
   if (current) return JXF_OK;
   batch_drop_groups(b);
   constexpr double kBytes = 70e6;
@@ -3383,7 +3391,11 @@ int batch_sweep_groups(jxf_batch3d* b) {
     for (auto& gr : b->groups) {
       std::vector<jxf_grid3d*> members;
       for (int k : gr.grids) members.push_back(b->grids[k]);
-      TRY(band_attach(members, b->band.band, b->device, &b->bytes, gr.band));
+      const int rc = band_attach(members, b->band.band, b->device, &b->bytes, gr.band);
+      if (rc != JXF_OK) {
+        batch_drop_groups(b);  // (a group left without its band would step as bare PEC)
+        return rc;
+      }
     }
   }
   return JXF_OK;
@@ -3635,6 +3647,7 @@ extern "C" int jxf_batch3d_step(jxf_batch3d* b, int32_t n_steps, int32_t use_gra
       return fail(JXF_ERR_INVALID, "a member grid's waveform table is too short");
   }
   DeviceGuard dg(b->device);
+  const AllocFault fault;
   int in_set = 0;
   if (b->tma) {
     in_set = b->grids[0]->cur;

@@ -1,0 +1,73 @@
+"""Batches on in-place passes whose first run meets a refused device
+allocation (``JXF_FAULT_ALLOC_AFTER``): the call raises, no grid has stepped,
+and a later call gives what a batch that never failed gives."""
+
+import numpy as np
+import pytest
+
+from gpu_helpers import to_np
+
+pytestmark = pytest.mark.gpu
+
+COMPS = ("ex", "ey", "ez", "hx", "hy", "hz")
+# more grids than one group holds
+SIZES = [(20, 24, 28), (33, 21, 16), (12, 40, 32), (24, 24, 24), (17, 16, 20), (30, 12, 36),
+         (18, 18, 16), (22, 26, 24), (14, 14, 12), (28, 20, 40)]
+
+
+def _batch():
+    from jaxphys_b200 import EMGrid3D
+    from jaxphys_b200.em.batch import FDTDBatch
+
+    grids = []
+    for i, size in enumerate(SIZES):
+        g = EMGrid3D(size=size, resolution=1.0, boundary="pec")
+        g.prepare()
+        g.set_field("ez", np.random.default_rng(i).standard_normal(size).astype(np.float32))
+        g.add_probe(tuple(s // 2 for s in size), "ey")
+        grids.append(g)
+    return grids, FDTDBatch(grids)
+
+
+def _fields(grids):
+    return [to_np(g.field(k)) for g in grids for k in COMPS]
+
+
+def _run_past_refusals(monkeypatch, grids, batch, steps):
+    """Run with 0, 1, 2, ... allocations allowed until one call succeeds."""
+    from jaxphys_b200 import SimulationError
+
+    before = _fields(grids)
+    for n in range(300):
+        monkeypatch.setenv("JXF_FAULT_ALLOC_AFTER", str(n))
+        try:
+            out = batch.run(steps)
+        except SimulationError as e:
+            assert "fault injection" in str(e)
+        else:
+            monkeypatch.delenv("JXF_FAULT_ALLOC_AFTER")
+            return n, out
+        monkeypatch.delenv("JXF_FAULT_ALLOC_AFTER")
+        for a, b in zip(_fields(grids), before):
+            assert np.array_equal(a, b), n
+    raise AssertionError("the run never succeeded")
+
+
+def test_refused_band_tables(cuda, monkeypatch):
+    """Every group keeps its band: none steps as bare PEC after a refusal."""
+    from jaxphys_b200.em.learned import default_band
+
+    monkeypatch.setenv("JXF_BATCH_LAUNCH", "sweep")
+    grids, batch = _batch()
+    batch.set_band(default_band())
+    refused, got = _run_past_refusals(monkeypatch, grids, batch, 9)
+    assert refused > 5  # the tables of both groups
+    ref_grids, ref = _batch()
+    ref.set_band(default_band())
+    want = ref.run(9)
+    for a, b in zip(got, want):
+        assert np.array_equal(to_np(a), to_np(b))
+    for a, b in zip(_fields(grids), _fields(ref_grids)):
+        assert np.array_equal(a, b)
+    batch.close()
+    ref.close()
