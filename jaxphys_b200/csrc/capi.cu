@@ -3684,6 +3684,8 @@ extern "C" int jxf_batch3d_step(jxf_batch3d* b, int32_t n_steps, int32_t use_gra
     // (launches of a group's whole run are queued one by one, with or without
     // use_graph: a graph of them all would hold 2 n nodes per group)
     TRY(batch_sweep_groups(b));
+    // (what can fail for want of memory comes before any group's first step)
+    for (jxf_grid3d* g : b->grids) TRY(build_sweep(g));
     for (auto& gr : b->groups) TRY(batch_sweep_group(b, gr, n_steps, false, st));
   } else if (!use_graph) {
     for (int k = 0; k < n_steps; ++k)

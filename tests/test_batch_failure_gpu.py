@@ -15,13 +15,15 @@ SIZES = [(20, 24, 28), (33, 21, 16), (12, 40, 32), (24, 24, 24), (17, 16, 20), (
          (18, 18, 16), (22, 26, 24), (14, 14, 12), (28, 20, 40)]
 
 
-def _batch():
-    from jaxphys_b200 import EMGrid3D
+def _batch(sources=False):
+    from jaxphys_b200 import EMGrid3D, PointSource3D
     from jaxphys_b200.em.batch import FDTDBatch
 
     grids = []
     for i, size in enumerate(SIZES):
         g = EMGrid3D(size=size, resolution=1.0, boundary="pec")
+        if sources:
+            g.add_source(PointSource3D(frequency=0.05 / g.default_dt(), position=(3, 4, 5)))
         g.prepare()
         g.set_field("ez", np.random.default_rng(i).standard_normal(size).astype(np.float32))
         g.add_probe(tuple(s // 2 for s in size), "ey")
@@ -64,6 +66,24 @@ def test_refused_band_tables(cuda, monkeypatch):
     assert refused > 5  # the tables of both groups
     ref_grids, ref = _batch()
     ref.set_band(default_band())
+    want = ref.run(9)
+    for a, b in zip(got, want):
+        assert np.array_equal(to_np(a), to_np(b))
+    for a, b in zip(_fields(grids), _fields(ref_grids)):
+        assert np.array_equal(a, b)
+    batch.close()
+    ref.close()
+
+
+def test_refused_source_lists(cuda, monkeypatch):
+    """No group has stepped when the source lists of a later one are refused."""
+    monkeypatch.setenv("JXF_BATCH_LAUNCH", "sweep")
+    grids, batch = _batch(sources=True)
+    refused, got = _run_past_refusals(monkeypatch, grids, batch, 9)
+    # (finished lists are kept, so each call gets further: the last ones into
+    # the second group)
+    assert refused >= 8
+    ref_grids, ref = _batch(sources=True)
     want = ref.run(9)
     for a, b in zip(got, want):
         assert np.array_equal(to_np(a), to_np(b))
