@@ -3671,6 +3671,7 @@ extern "C" int jxf_batch3d_step(jxf_batch3d* b, int32_t n_steps, int32_t use_gra
   }
   const size_t need = (size_t)n_steps * std::max(b->n_probes, 1);
   if (need > b->probe_cap) {
+    b->probe_cap = 0;  // (until the larger buffer is there)
     dfree(b->d_probe_buf);
     TRY(dmalloc(&b->d_probe_buf, need, &b->bytes));
     b->probe_cap = need;

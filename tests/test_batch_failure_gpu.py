@@ -91,3 +91,25 @@ def test_refused_source_lists(cuda, monkeypatch):
         assert np.array_equal(a, b)
     batch.close()
     ref.close()
+
+
+@pytest.mark.parametrize("launch", ["sweep", "0,8"])
+def test_refused_longer_probe_buffer(cuda, monkeypatch, launch):
+    """A refused buffer for a longer run does not cost the shorter runs after
+    it their probe rows."""
+    from jaxphys_b200 import SimulationError
+
+    monkeypatch.setenv("JXF_BATCH_LAUNCH", launch)
+    grids, batch = _batch(sources=True)
+    first = batch.run(4)
+    monkeypatch.setenv("JXF_FAULT_ALLOC_AFTER", "0")
+    with pytest.raises(SimulationError, match="fault injection"):
+        batch.run(9)
+    monkeypatch.delenv("JXF_FAULT_ALLOC_AFTER")
+    second = batch.run(3)
+    ref_grids, ref = _batch(sources=True)
+    want = ref.run(7)
+    for a, b, c in zip(first, second, want):
+        assert np.array_equal(np.vstack([to_np(a), to_np(b)]), to_np(c))
+    batch.close()
+    ref.close()
