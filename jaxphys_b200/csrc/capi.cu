@@ -3541,6 +3541,7 @@ int batch_tma_tune(jxf_batch3d* b, int in_set, cudaStream_t st) {
       }
   }
   b->sweep = sweep_ms < best;
+  if (!b->sweep) batch_drop_groups(b);  // (with a band: its tables, which lockstep has its own of)
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   b->cfg = bc;

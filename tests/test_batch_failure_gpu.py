@@ -1,6 +1,7 @@
 """Batches on in-place passes whose first run meets a refused device
 allocation (``JXF_FAULT_ALLOC_AFTER``): the call raises, no grid has stepped,
-and a later call gives what a batch that never failed gives."""
+and a later call gives what a batch that never failed gives.  And a batch that tries
+the passes but keeps lockstep holds one set of band tables."""
 
 import numpy as np
 import pytest
@@ -113,3 +114,44 @@ def test_refused_longer_probe_buffer(cuda, monkeypatch, launch):
         assert np.array_equal(np.vstack([to_np(a), to_np(b)]), to_np(c))
     batch.close()
     ref.close()
+
+
+def test_lockstep_holds_one_set_of_band_tables(cuda, monkeypatch):
+    """Two batches in turn on grids above the L2, where lockstep is faster:
+    one tunes (and so tries the passes), one is pinned to the shape found.  A
+    second set of band tables would be 32 bytes for each of the outer cells."""
+    import gc
+
+    import torch
+
+    from jaxphys_b200 import EMGrid3D
+    from jaxphys_b200.em.batch import FDTDBatch
+    from jaxphys_b200.em.learned import default_band
+
+    grids = [EMGrid3D(size=(256, 256, 256), resolution=1.0, boundary="pec") for _ in range(3)]
+    for g in grids:
+        g.prepare()
+    band = default_band()
+    second = 3 * 32 * (256**3 - 254**3)
+
+    def used():
+        gc.collect()
+        torch.cuda.synchronize()
+        free, total = torch.cuda.mem_get_info(0)
+        return total - free
+
+    taken = []
+    for _ in range(2):
+        batch = FDTDBatch(grids)
+        batch.set_band(band)
+        before = used()
+        batch.run(2, use_graph=False)
+        taken.append(used() - before)
+        shape = batch.launch()
+        if len(taken) == 1 and shape["tma_config"] < 0:
+            pytest.skip("the passes were faster here")
+        monkeypatch.setenv("JXF_BATCH_LAUNCH",
+                           f"{shape['tma_config']},{shape['x_chunk']},{shape['axis_split']}")
+        batch.close()
+        batch = None
+    assert taken[0] - taken[1] < second / 2, (taken, second)
