@@ -3343,49 +3343,87 @@ void batch_drop_groups(jxf_batch3d* b) {
   b->groups.clear();
 }
 
+// The kernels that grid k of a batch steps with.
+SweepGroupKernel batch_sweep_kernel(const jxf_batch3d* b, int k) {
+  const jxf_grid3d* g = b->grids[k];
+  return sweep_kernels(g->mode, g->kappa, g->cb != nullptr, g->d.nz).group_e;
+}
+
+// Bytes of a grid's fields, psi and permittivity factors (one buffer set).
+double sweep_bytes(const jxf_grid3d* g) {
+  double c = (double)g->n * (g->cb ? 7 : 6);
+  for (int q = 0; q < PSI_COUNT; ++q) c += (double)psi_size(g, q);
+  return 4.0 * c;
+}
+
 // Groups: grids that run the same kernel, largest first into the first group
 // with room.  70 MB of state is the most that keeps the speed of a resident
 // grid (128^3 CPML: 70 MB, 87 Gcell/s; 160^3: 135 MB, 70 Gcell/s).
+std::vector<std::vector<int>> batch_sweep_plan(const jxf_batch3d* b) {
+  constexpr double kBytes = 70e6;
+  const int n = (int)b->grids.size();
+  std::vector<double> bytes(n);
+  for (int k = 0; k < n; ++k) bytes[k] = sweep_bytes(b->grids[k]);
+  std::vector<int> order(n);
+  std::iota(order.begin(), order.end(), 0);
+  std::stable_sort(order.begin(), order.end(), [&](int u, int v) { return bytes[u] > bytes[v]; });
+  std::vector<std::vector<int>> groups;
+  std::vector<double> fill;
+  for (int k : order) {
+    size_t i = 0;
+    while (i < groups.size() &&
+           (fill[i] + bytes[k] > kBytes || groups[i].size() >= SWEEP_GROUP ||
+            batch_sweep_kernel(b, groups[i][0]) != batch_sweep_kernel(b, k)))
+      ++i;
+    if (i == groups.size()) {
+      groups.emplace_back();
+      fill.push_back(0.0);
+    }
+    groups[i].push_back(k);
+    fill[i] += bytes[k];
+  }
+  return groups;
+}
+
+// Whether groups beat lockstep for a batch whose grids have one buffer set, so
+// that neither can be tried without stepping it.  A group's launches take a
+// few microseconds a step however small its grids are, lockstep pays that once
+// for the whole batch; against it stand the microseconds a step that a cell
+// costs less in a group.  Fitted on one B200 to 9 to 160 grids of sides 9 to
+// 57 (nz % 4 != 0, 400 steps a run; us a step, lockstep and groups): 64 PEC
+// grids of 17^3 19 and 49, of 33^3 53 and 81, of 49^3 (180 MB, out of the L2)
+// 212 and 167; 64 CPML grids of 17^3 32 and 67, of 25^3 63 and 91, of 33^3 133
+// and 110; 64 grids behind the band of 17^3 56 and 154, of 57^3 822 and 755.
+// The faster one, or one within 15 % of it, is taken for all 240 of them.
+bool batch_sweep_pays(const jxf_batch3d* b) {
+  const bool cpml = b->mode == MODE_CPML, band = b->band.band != nullptr;
+  const double groups = (double)batch_sweep_plan(b).size();
+  double bytes = 0.0, gain = 0.0;
+  for (const jxf_grid3d* g : b->grids) bytes += sweep_bytes(g);
+  const bool past_l2 = bytes > (band ? 100e6 : 70e6);
+  for (const jxf_grid3d* g : b->grids) {
+    const bool pairs = g->d.nz % 2 == 0 && !band;  // two cells a thread
+    const double cell = cpml ? 38e-6 : past_l2 ? (pairs ? 15e-6 : 10e-6) : (pairs ? 5.5e-6 : 0.0);
+    gain += cell * (double)g->n;
+  }
+  // (one group: fewer launches than lockstep has)
+  const double cost = cpml ? 8.5 * groups - 10.0 : band ? 16.0 * groups - 18.0 : 4.5 * groups - 6.0;
+  return gain > cost;
+}
+
 int batch_sweep_groups(jxf_batch3d* b) {
-  auto kernel_of = [&](int k) {
-    const jxf_grid3d* g = b->grids[k];
-    return sweep_kernels(g->mode, g->kappa, g->cb != nullptr, g->d.nz).group_e;
-  };
   // (a permittivity map set or dropped since changes a grid's kernel)
   bool current = !b->groups.empty();
   for (const auto& gr : b->groups) {
     current = current && gr.band.band == b->band.band;
-    for (int k : gr.grids) current = current && kernel_of(k) == kernel_of(gr.grids[0]);
+    for (int k : gr.grids)
+      current = current && batch_sweep_kernel(b, k) == batch_sweep_kernel(b, gr.grids[0]);
   }
   if (current) return JXF_OK;
   batch_drop_groups(b);
-  constexpr double kBytes = 70e6;
-  const int n = (int)b->grids.size();
-  std::vector<double> bytes(n);
-  for (int k = 0; k < n; ++k) {
-    const jxf_grid3d* g = b->grids[k];
-    double c = (double)g->n * (g->cb ? 7 : 6);
-    if (g->mode == MODE_CPML)
-      c += 4.0 * ((double)g->L[0] * g->d.ny * g->d.nz + (double)g->d.nx * g->L[1] * g->d.nz +
-                  (double)g->d.nx * g->d.ny * g->L[2]);
-    bytes[k] = 4.0 * c;
-  }
-  std::vector<int> order(n);
-  std::iota(order.begin(), order.end(), 0);
-  std::stable_sort(order.begin(), order.end(), [&](int u, int v) { return bytes[u] > bytes[v]; });
-  std::vector<double> fill;
-  for (int k : order) {
-    size_t i = 0;
-    while (i < b->groups.size() &&
-           (fill[i] + bytes[k] > kBytes || b->groups[i].grids.size() >= SWEEP_GROUP ||
-            kernel_of(b->groups[i].grids[0]) != kernel_of(k)))
-      ++i;
-    if (i == b->groups.size()) {
-      b->groups.emplace_back();
-      fill.push_back(0.0);
-    }
-    b->groups[i].grids.push_back(k);
-    fill[i] += bytes[k];
+  for (auto& grids : batch_sweep_plan(b)) {
+    b->groups.emplace_back();
+    b->groups.back().grids = std::move(grids);
   }
   if (b->band.band) {
     for (auto& gr : b->groups) {
@@ -3660,8 +3698,11 @@ extern "C" int jxf_batch3d_step(jxf_batch3d* b, int32_t n_steps, int32_t use_gra
     if (!b->tuned) TRY(batch_tma_tune(b, in_set, (cudaStream_t)stream));
   } else if (!b->tuned) {
     // (a caller who asked for the generic path gets its per-cell kernels)
+    const char* forced = std::getenv("JXF_BATCH_LAUNCH");
     b->tuned = true;
-    b->sweep = batch_can_sweep(b);
+    b->sweep = batch_can_sweep(b) &&
+               ((forced && std::strcmp(forced, "sweep") == 0) || batch_sweep_pays(b));
+    if (!b->sweep) batch_drop_groups(b);
   }
   TRY(batch_refresh(b));
   if (b->band.band && !b->sweep && b->band.tiles == 0) {
@@ -4441,6 +4482,7 @@ int jxf_batch3d_set_band(jxf_batch3d* b, jxf_band* m) {
   }
   band_release(b->band);
   batch_drop_groups(b);
+  if (!b->tma) b->tuned = false;  // (the band weighs in its choice)
   if (!m) return JXF_OK;
   // (its tables are built by the first run, for all grids or group by group)
   TRY(band_check(b->grids, m, b->device));
