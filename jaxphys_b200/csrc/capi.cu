@@ -1812,6 +1812,7 @@ int jxf_grid3d_set_blocked(jxf_grid3d* g, int32_t cfg, int32_t x_chunk) {
 int jxf_grid3d_set_axis_split(jxf_grid3d* g, int32_t on) {
   if (!g) return fail(JXF_ERR_INVALID, "null handle");
   g->axis_split = on ? 1 : 0;
+  if (g->cfg >= 0) g->sweep = false;  // (the split is of TMA launches)
   return JXF_OK;
 }
 
