@@ -1122,6 +1122,15 @@ bool sweep_ok(const jxf_grid3d* g) {
          (long long)g->d.nx * g->d.ny * g->L[2] < (1LL << 31);
 }
 
+// Grids that always step in sweeps: those the TMA kernels do not take (odd
+// rows, periodic), unless the caller asked for the per-cell kernels.
+bool sweep_always(const jxf_grid3d* g) {
+  return g->path == JXF_PATH_GENERIC && g->d.path == JXF_PATH_AUTO && sweep_ok(g);
+}
+
+// (a TMA-path grid has been through ensure_tma_ready)
+bool steps_by_sweep(const jxf_grid3d* g) { return g->sweep || sweep_always(g); }
+
 // The work split of a plane for kernels of v0 / v1 cells per thread outside /
 // inside the z slabs.  margin: cells on the inner side of each psi slab that
 // belong to its regions too.
@@ -1762,7 +1771,7 @@ int jxf_grid3d_get_info(const jxf_grid3d* g, jxf_grid3d_info* out) {
                   (g->n_tb_shell_ax[4] > 0 ? 1 : 0) + (g->n_tb_shell_ax[5] > 0 ? 1 : 0);
   else
     out->blocked_kernels_per_pass = 0;
-  if (g->sweep || (g->path == JXF_PATH_GENERIC && sweep_ok(g)))
+  if (steps_by_sweep(g))
     out->kernels_per_step = 2;
   else if (g->path == JXF_PATH_GENERIC)
     out->kernels_per_step = 2 + (g->n_cells > 0 ? 1 : 0);
@@ -1994,10 +2003,6 @@ static int check_waves3d(const jxf_grid3d* g, long long n_steps) {
   return JXF_OK;
 }
 
-// (a TMA-path grid has been through ensure_tma_ready)
-static bool steps_by_sweep(const jxf_grid3d* g) {
-  return g->sweep || (g->path == JXF_PATH_GENERIC && sweep_ok(g));
-}
 
 // Floats of a snapshot (H and the E psi after a step), and one at `base`.
 static size_t snap_floats(const jxf_grid3d* g) {

@@ -44,3 +44,33 @@ def test_pinned_launch_ends_the_passes(cuda, call):
     assert np.array_equal(np.vstack(traces), to_np(ref.run(15)))
     for a, b in zip(grid_fields(g), grid_fields(ref)):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("boundary", ["cpml", "absorbing", "pec", "periodic"])
+def test_generic_path_runs_the_per_cell_kernels(cuda, boundary):
+    """Three launches a step (H, E, sources), whole grids of every boundary."""
+    for size in (SIZE, (11, 14, 13)):
+        g, ref = _grid("generic", boundary, size), _grid("auto", boundary, size)
+        got = np.vstack([to_np(g.run(9)), to_np(g.run(6))])
+        want = to_np(ref.run(15))
+        assert g.kernels_per_step() == 3 and ref.kernels_per_step() == 2
+        assert np.array_equal(got, want) and np.abs(want).max() > 0
+        for a, b in zip(grid_fields(g), grid_fields(ref)):
+            assert np.array_equal(a, b)
+
+
+def test_gradient_of_a_generic_grid(cuda):
+    """The adjoint of a per-cell grid recomputes with the same kernels."""
+    import torch
+
+    from jaxphys_b200.em.adjoint import probe_traces
+
+    grads = []
+    for path in ("generic", "auto"):
+        g = _grid(path, "cpml", (12, 13, 14), eps=False)
+        e = torch.tensor(smooth_eps((12, 13, 14), 1.0, 4.0, seed=5), dtype=torch.float32,
+                         device=cuda, requires_grad=True)
+        (probe_traces(g, e, 30) ** 2).sum().backward()
+        grads.append(to_np(e.grad))
+        assert g.kernels_per_step() == (3 if path == "generic" else 2)
+    assert np.array_equal(grads[0], grads[1]) and np.abs(grads[0]).max() > 0
