@@ -1946,6 +1946,8 @@ int jxf_grid3d_set_sources(jxf_grid3d* g, int32_t n, const int64_t* cell, const 
   g->built_cfg = -1;
   g->tb_built_cfg = -1;
   g->sweep_built = false;
+  // (here and not in the next step, which a caller may capture into a graph)
+  if (sweep_always(g)) TRY(build_sweep(g));
   return JXF_OK;
 }
 
