@@ -2572,9 +2572,18 @@ bool block2d_choose(const jxf_grid2d* g, int n, int* cfg, int* steps) {
   return best < 1e30;
 }
 
-bool block2d_ready(jxf_grid2d* g) {
+// The second buffer set, allocated on first use.  Not while the caller captures
+// the stream into a graph, where an allocation would end the capture: such a
+// call takes the one-step kernels.
+bool block2d_ready(jxf_grid2d* g, cudaStream_t st) {
   if (g->no_f2) return false;
   if (g->f2[0]) return true;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &capture) != cudaSuccess ||
+      capture != cudaStreamCaptureStatusNone) {
+    (void)cudaGetLastError();
+    return false;
+  }
   for (int k = 0; k < 3; ++k)
     if (dmalloc(&g->f2[k], (size_t)g->n, &g->bytes) != JXF_OK) {
       (void)cudaGetLastError();
@@ -2837,7 +2846,7 @@ int jxf_grid2d_step(jxf_grid2d* g, int32_t n_steps, void* stream) {
   Step2D p = step2d_params(g);
   // one step: in place (a launch of several would have to copy back)
   int cfg = 0, steps = 0, set = 0;
-  if (n_steps >= 2 && block2d_choose(g, n_steps, &cfg, &steps) && block2d_ready(g)) {
+  if (n_steps >= 2 && block2d_choose(g, n_steps, &cfg, &steps) && block2d_ready(g, st)) {
     TRY(block2d_advance(g, p, cfg, steps, n_steps, true, nullptr, &set, st));
     return block2d_settle(g, set, st);
   }
@@ -2864,7 +2873,7 @@ int jxf_grid2d_run(jxf_grid2d* g, int32_t n_steps, int32_t save_every, int64_t n
   // the launch shape follows from the usual run between two frames
   int cfg = 0, steps = 0;
   const int usual = n_frames > 1 ? save_every : n_steps;
-  const bool blocked = block2d_choose(g, usual, &cfg, &steps) && block2d_ready(g);
+  const bool blocked = block2d_choose(g, usual, &cfg, &steps) && block2d_ready(g, st);
   for (int64_t k = 0; k <= n_frames; ++k) {
     const bool save = k < n_frames;
     const int n = (int)(first + (save ? 1 + k * (int64_t)save_every : n_steps) - g->step);

@@ -6,7 +6,7 @@ gives outside one."""
 import numpy as np
 import pytest
 
-from gpu_helpers import grid_fields, to_np
+from gpu_helpers import grid_fields
 
 pytestmark = pytest.mark.gpu
 
@@ -49,3 +49,37 @@ def test_first_steps_of_a_3d_grid(cuda, size, boundary, sources):
     step(ref)
     for a, b in zip(grid_fields(g), grid_fields(ref)):
         assert np.array_equal(a, b) and np.abs(b).max() > 0
+
+
+@pytest.mark.parametrize("boundary", ["absorbing", "periodic", "reflecting"])
+def test_first_steps_of_a_2d_grid(cuda, boundary):
+    """And the steps after those, outside a graph: several per launch."""
+    from jaxphys_b200 import EMGrid, PlaneWave, Wall
+    from jaxphys_b200 import _native as nat
+
+    lib = nat.load()
+
+    def grid():
+        g = EMGrid(size=(37, 45), boundary=boundary, pml_layers=4)
+        g.add_source(PlaneWave(frequency=2e9, y=7))
+        g.add_conductor(Wall(y=20, gap_start=10, gap_end=18))
+        g._prepare(g.default_dt(), 0.0, 2 * STEPS)
+        return g
+
+    def step(g):
+        nat.check(lib.jxf_grid2d_step(g._h, STEPS, nat.stream_handle()), "step")
+
+    def fields(g):
+        out = np.empty((3,) + g.size, dtype=np.float32)
+        for c in range(3):
+            nat.check(lib.jxf_grid2d_get_field(g._h, c, out[c].ctypes.data, 1,
+                                               nat.stream_handle()), "get")
+        return out
+
+    g, ref = grid(), grid()
+    _capture_and_replay(lambda: step(g))
+    step(ref)
+    assert np.array_equal(fields(g), fields(ref))
+    step(g)
+    step(ref)
+    assert np.array_equal(fields(g), fields(ref)) and np.abs(fields(g)).max() > 0
