@@ -174,9 +174,10 @@ int jxf_grid3d_run(jxf_grid3d* g, int32_t n_steps, int32_t save_every, int64_t n
  * into probe_out (device [n_steps][n_probes], may be NULL) and keeping a
  * checkpoint of the full state every checkpoint_every steps (<= 0: the H and
  * psi_E snapshots of as many last steps as fit a sixteenth of the device's
- * memory and an eighth of what is free beside the gradient's other buffers are
- * kept, and the steps before them get checkpoints every ceil(sqrt) of their
- * number).
+ * memory, over all grids of the process, and an eighth of what is free beside
+ * the gradient's other buffers are kept, and the steps before them get
+ * checkpoints every ceil(sqrt) of their number).  The buffers stay with the
+ * grid for its next gradient.
  * jxf_grid3d_adjoint_backward: probe_grad = dJ/d(probe_out) (device
  * [n_steps][n_probes]); writes dJ/d(eps_r) (device float32 [nx*ny*nz]).
  * Recomputes each checkpointed segment forward (one segment of H and psi_E
@@ -186,6 +187,10 @@ int jxf_grid3d_adjoint_forward(jxf_grid3d* g, int32_t n_steps, int32_t checkpoin
                                float* probe_out, void* stream);
 int jxf_grid3d_adjoint_backward(jxf_grid3d* g, const float* probe_grad, float* grad_eps,
                                 void* stream);
+/* Give back the device memory of the gradient (checkpoints, snapshots, adjoint
+ * fields); it also goes with the grid.  Waits for work in flight.  The next
+ * gradient starts with jxf_grid3d_adjoint_forward. */
+int jxf_grid3d_adjoint_release(jxf_grid3d* g);
 
 /* Decomposition of one grid along x over several processes (one per GPU;
  * the reference runs a single device).  jxf_grid3d_create_slab makes the

@@ -247,6 +247,7 @@ struct BandTables {
 
 struct jxf_batch3d;
 namespace {
+void adjoint_free(jxf_grid3d* g);
 void batch_drop_groups(jxf_batch3d* b);
 int band_launch(const BandTables& t, cudaStream_t st, int set = 0, bool pdl = false);
 int band_attach(const std::vector<jxf_grid3d*>& grids, jxf_band* m, int device, int64_t* tally,
@@ -1721,11 +1722,7 @@ int jxf_grid3d_destroy(jxf_grid3d* g) {
   dfree(g->d_sw_ptr);
   dfree(g->d_sw_cells);
   dfree(g->d_sw_terms);
-  dfree(g->adj_ck);
-  dfree(g->adj_sg);
-  dfree(g->adj_kp);
-  dfree(g->adj_l);
-  dfree(g->adj_g);
+  adjoint_free(g);
   dfree(g->d_wave);
   dfree(g->d_probe_cell);
   dfree(g->d_probe_comp);
@@ -4527,6 +4524,14 @@ int jxf_grid3d_set_band(jxf_grid3d* g, jxf_band* m) {
 
 namespace {
 
+// Bytes of kept snapshots on every device, over all grids of the process: what
+// the library may hold for them is bounded once, not per grid.
+struct KeptBytes {
+  std::mutex mu;
+  std::map<int, size_t> on;  // device -> bytes
+};
+KeptBytes g_kept;
+
 template <class T>
 int ensure_buf(T** p, size_t* cap, size_t count, int64_t* tally) {
   if (*cap >= count && *p) return JXF_OK;
@@ -4535,6 +4540,24 @@ int ensure_buf(T** p, size_t* cap, size_t count, int64_t* tally) {
   TRY(dmalloc(p, count, tally));
   *cap = count;
   return JXF_OK;
+}
+
+// Gives back every buffer of the gradient (a forward call takes them again).
+void adjoint_free(jxf_grid3d* g) {
+  if (g->adj_kp_cap > 0) {
+    std::lock_guard<std::mutex> lk(g_kept.mu);
+    g_kept.on[g->d.device] -= 4 * g->adj_kp_cap;
+  }
+  g->bytes -= 4 * (int64_t)(g->adj_ck_cap + g->adj_sg_cap + g->adj_kp_cap + g->adj_l_cap) +
+              8 * (int64_t)g->adj_g_cap;
+  dfree(g->adj_ck);
+  dfree(g->adj_sg);
+  dfree(g->adj_kp);
+  dfree(g->adj_l);
+  dfree(g->adj_g);
+  g->adj_ck_cap = g->adj_sg_cap = g->adj_kp_cap = g->adj_l_cap = g->adj_g_cap = 0;
+  g->adj_kp_want = 0;
+  g->adj_n = 0;
 }
 
 // Several device-to-device copies of float arrays in one launch (the
@@ -4617,8 +4640,9 @@ extern "C" int jxf_grid3d_adjoint_forward(jxf_grid3d* g, int32_t n_steps,
   for (int k = 0; k < PSI_COUNT; ++k) state += psi_size(g, k);
   if (g->path == JXF_PATH_TMA) TRY(ensure_tma_ready(g, st));
   // Where the caller leaves the memory to the library, the snapshots of as
-  // many last steps as fit a sixteenth of the device (and an eighth of what is
-  // free of it) are kept, and only the steps before them are recomputed: a
+  // many last steps as fit a sixteenth of the device (over all grids of the
+  // process, so that many of them leave a caller the rest; and an eighth of what
+  // is free) are kept, and only the steps before them are recomputed: a
   // recomputed step costs as much as a forward one (96^3, 2000 steps, 650 of
   // them kept in 11 GB: 104.8 ms a gradient against 116.7; 48^3, 300 steps, all
   // kept: 5.96 against 8.60).
@@ -4640,11 +4664,16 @@ extern "C" int jxf_grid3d_adjoint_forward(jxf_grid3d* g, int32_t n_steps,
       // checkpoints, a segment's snapshots, adjoint fields and two psi sets,
       // dJ/dcb in FP64
       const size_t rest = 4 * ((kk + 1) * state + kk * snap + 2 * state);
-      const size_t may = std::min(total_b / 16, (free_b > rest ? free_b - rest : 0) / 8) / 4;
+      std::lock_guard<std::mutex> lk(g_kept.mu);
+      size_t& kept = g_kept.on[g->d.device];
+      kept -= 4 * g->adj_kp_cap;  // (of other grids)
+      const size_t room = total_b / 16 > kept ? total_b / 16 - kept : 0;
+      const size_t may = std::min(room, (free_b > rest ? free_b - rest : 0) / 8) / 4;
       const size_t get = std::min(want, may / snap * snap);
       if (get > g->adj_kp_cap &&
           ensure_buf(&g->adj_kp, &g->adj_kp_cap, get, &g->bytes) != JXF_OK)
         (void)cudaGetLastError();  // no room: recompute
+      kept += 4 * g->adj_kp_cap;
       g->adj_kp_want = want;
     }
     keep = (int)std::min<size_t>(most, g->adj_kp_cap / snap);
@@ -4788,6 +4817,13 @@ extern "C" int jxf_grid3d_adjoint_backward(jxf_grid3d* g, const float* probe_gra
                                          (long long)n);
   CUDA_TRY(cudaGetLastError());
   return jxf_grid3d_reset(g, stream);  // leave the grid at its initial state
+}
+
+extern "C" int jxf_grid3d_adjoint_release(jxf_grid3d* g) {
+  if (!g) return fail(JXF_ERR_INVALID, "null handle");
+  DeviceGuard dg(g->d.device);
+  adjoint_free(g);
+  return JXF_OK;
 }
 
 // ---------------------------------------------------------------------------

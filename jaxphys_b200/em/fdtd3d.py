@@ -480,8 +480,9 @@ class EMGrid3D:
         """Extension: reset, run ``n_steps`` keeping what
         :meth:`adjoint_backward` needs: a checkpoint every ``checkpoint_every``
         steps, or by default the snapshots of as many last steps as fit a
-        sixteenth of the device and sqrt(T) checkpoints of the others; returns
-        the probe traces (n_steps, P)."""
+        sixteenth of the device (over all grids of the process) and sqrt(T)
+        checkpoints of the others; returns the probe traces (n_steps, P).
+        The memory stays with the grid: :meth:`adjoint_release`."""
         import torch
 
         if self._h is None:
@@ -509,6 +510,13 @@ class EMGrid3D:
                                                          nat.stream_handle()),
                   "jxf_grid3d_adjoint_backward")
         return out
+
+    def adjoint_release(self) -> None:
+        """Extension: give back the device memory that the gradients of this
+        grid hold between calls (the next ``adjoint_forward`` takes it again)."""
+        if self._h is not None:
+            nat.check(nat.load().jxf_grid3d_adjoint_release(self._h),
+                      "jxf_grid3d_adjoint_release")
 
     def step(self, n: int = 1) -> None:
         """Extension: advance ``n`` steps without probe recording."""
