@@ -59,6 +59,7 @@ WORKLOADS = {
     "c5": (64, 1000, 3, "batch64-sides48to160-eps1to6-dipoles-learnedband3-vs-cpml10"),
 }
 BAND_WEIGHTS = ROOT / "jaxphys_b200" / "em" / "band_weights.npz"
+L2_BYTES = 126e6
 
 
 
@@ -113,6 +114,20 @@ def psi_bytes_per_cell(n: int, pml: int) -> float:
     P = pml + 1
     frac = min(2 * P, n) / n
     return 12 * frac * 8.0
+
+
+def step_roofline(n: int, pml: int, with_eps: bool, in_place: bool):
+    """What bounds a CPML step of an n^3 grid, and the bytes a cell it moves
+    there.  One pass (marching, or blocked per step) reads and writes six
+    fields through HBM; the two in-place passes read each other's fields too
+    (H: 6 in, 3 out; E: 6 in, 3 out), through the L2 where one set of fields
+    and psi stays in it."""
+    psi = psi_bytes_per_cell(n, pml)
+    eps = 4.0 if with_eps else 0.0
+    if not in_place:
+        return "hbm", 48.0 + eps + psi
+    state = n ** 3 * (24.0 + eps + psi / 2)
+    return ("l2" if state < L2_BYTES else "hbm"), 72.0 + eps + psi
 
 
 def measured_peaks():
@@ -307,15 +322,16 @@ def run_ours(args, world, rank, local, pg, workload=None, steps=None, warmup=Non
     value = updates / (total_ms * 1e-3) / 1e9
     e2e_value = updates / (e2e_ms * 1e-3) / 1e9
 
-    # ---- roofline of the dominant kernel (the fused TMA step)
+    # ---- roofline of the step's kernels
     info = g.info()
     # one leapfrog step = the step launch(es) of one time step (the probe
     # gather that ends each run is < 0.1 % of it)
     per_launch_ms = statistics.mean(kern_ms) / nsteps
-    b_cell = 52.0 + psi_bytes_per_cell(n, pml) if eps is not None else 48.0 + psi_bytes_per_cell(n, pml)
+    bound, b_cell = step_roofline(n, pml, eps is not None, info["tma_config"] < 0)
     bytes_per_launch = cells * b_cell
     achieved = bytes_per_launch / (per_launch_ms * 1e-3) / 1e9
-    peak, peak_kind = measured_peaks()
+    # (there is no measured peak for the L2, so no fraction either)
+    peak, peak_kind = measured_peaks() if bound == "hbm" else (None, None)
     launch = {"tma_config": info["tma_config"], "x_chunk": info["x_chunk"],
               "axis_split": info["axis_split"], "blocked_config": info["blocked_config"],
               "blocked_x_chunk": info["blocked_x_chunk"]}
@@ -351,9 +367,9 @@ def run_ours(args, world, rank, local, pg, workload=None, steps=None, warmup=Non
                    "parallelism": f"independent grid per GPU x{world}"},
         "e2e": {"value": round(e2e_value, 3), "unit": "Gcell/s", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h},
-        "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-                     "frac": round(achieved / peak, 4), "traffic": traffic,
-                     "peak_source": peak_kind, "bytes_per_cell_update": round(b_cell, 2),
+        "roofline": {"bound": bound, "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
+                     "frac": None if peak is None else round(achieved / peak, 4),
+                     "traffic": traffic, "peak_source": peak_kind, "bytes_per_cell_update": round(b_cell, 2),
                      "kernel": ("k3d_tb2 two-level blocked pass (every launch of a pass), "
                                 "per leapfrog step" if blocked else
                                 "k3d_tma step (every launch of one leapfrog step)"
@@ -514,12 +530,14 @@ def run_batch(args, world, rank, local, pg, steps=None, warmup=None, reflection=
     lr = results["learned"]
     peak, peak_kind = measured_peaks()
     # algorithmic bytes of one leapfrog step of the learned batch: the Yee
-    # update (6 components read + written, eps read: 52 B per cell) and the
-    # band (outer cells: 24 B stencil centre read, 24 B correction written
-    # and read back, 24 B field read-modify-write: 120 B per outer cell)
+    # update (6 components read + written, eps read: 52 B per cell; in-place
+    # passes 76 B, from the L2) and the band (outer cells: 24 B stencil centre
+    # read, 24 B correction written and read back, 24 B field
+    # read-modify-write: 120 B per outer cell)
     outer = sum(int(np.prod(np.array(c.size) + 6)) - int(np.prod(np.array(c.size) + 4))
                 for c in all_cases)
-    step_bytes = lr["grid_cells"] * 52.0 + outer * 120.0
+    grouped = lr.get("launch", {}).get("tma_config", -1) < 0
+    step_bytes = lr["grid_cells"] * (76.0 if grouped else 52.0) + outer * 120.0
     # per GPU (the batch is split over the ranks)
     achieved = step_bytes / world / (lr["ms_per_step"] / nsteps * 1e-3) / 1e9
     line = {
@@ -538,15 +556,16 @@ def run_batch(args, world, rank, local, pg, steps=None, warmup=None, reflection=
         "config": {"workload": wname, "grids": n_grids, "interior_cells": interior_total,
                    "leapfrog_steps_per_step": nsteps, "band_layers": BAND_LAYERS,
                    "l2": "inputs larger than L2 (>= 360 MB of fields)",
-                   "path": ("tma (persistent batch launch)"
-                            if lr.get("launch", {}).get("tma_config", -1) >= 0
-                            else "in-place passes, group by group"),
+                   "path": ("in-place passes, group by group" if grouped
+                            else "tma (persistent batch launch)"),
                    "launch": lr.pop("launch", None),
                    "parallelism": f"the {n_grids} grids bin-packed by cell count over {world} GPU(s)"},
         "compare": {k: results[k] for k in ("cpml10", "cpml4", "pec") if k in results},
         "reflection_db": refl,
-        "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-                     "frac": round(achieved / peak, 4), "traffic": None, "peak_source": peak_kind,
+        "roofline": {"bound": "l2" if grouped else "hbm", "achieved": round(achieved, 1),
+                     "peak": None if grouped else peak, "unit": "GB/s",
+                     "frac": None if grouped else round(achieved / peak, 4), "traffic": None,
+                     "peak_source": None if grouped else peak_kind,
                      "kernel": "whole learned-batch leapfrog step (Yee + band)"},
         "gpu_launches": launches,
         "clocks": lr.pop("clocks"),
