@@ -16,9 +16,10 @@ permittivity map goes in from pinned host memory, the probe traces come
 back to the host) every step.  L2 is flushed (a 256 MiB write) between timed
 steps; each step is bracketed by CUDA events on the launching stream.
 
---impl reference times the CPU restatement of the reference algorithm
-(oracle/cpu_fdtd.c, FP64, every host thread) on a bounded sample of the
-same workload; under torchrun only rank 0 runs it.
+--impl reference prints why the reference itself cannot run here (it needs
+JAX).  `cpu_baseline` in our own line is the CPU restatement of its step
+(oracle/cpu_fdtd.c, FP64, every host thread) on a bounded sample of the same
+workload.
 
 With --gpus N > 1 (torchrun, one process per GPU) every rank runs its own
 independent grid of the same workload (grids do not exchange data), so the
@@ -650,7 +651,7 @@ def run_adjoint(args, world, rank, local, pg, steps=None, warmup=None, emit=True
     return line
 
 
-def cpu_baseline(workload: str, budget_s: float = 10.0, steps: int | None = None):
+def cpu_baseline(workload: str, budget_s: float = 10.0):
     """The FP64 C restatement of the reference step on every host thread, on a
     bounded sample (a prefix of the workload's leapfrog steps)."""
     from oracle import ref_numpy as rn
@@ -666,11 +667,10 @@ def cpu_baseline(workload: str, budget_s: float = 10.0, steps: int | None = None
                      probes=[p + (2,) for p in probes])
     o = Oracle3DC(spec, dt=dt)
     o.run(2)
-    if steps is None:
-        t0 = time.perf_counter()
-        o.run(4)
-        per = (time.perf_counter() - t0) / 4
-        steps = max(4, min(nsteps, int(budget_s / max(per, 1e-6))))
+    t0 = time.perf_counter()
+    o.run(4)
+    per = (time.perf_counter() - t0) / 4
+    steps = max(4, min(nsteps, int(budget_s / max(per, 1e-6))))
     t0 = time.perf_counter()
     o.run(steps)
     el = time.perf_counter() - t0
@@ -681,57 +681,15 @@ def cpu_baseline(workload: str, budget_s: float = 10.0, steps: int | None = None
             "seconds": round(el, 4)}
 
 
-def run_reference(args, world, rank):
-    """The reference arm: the CPU restatement of the reference step (FP64 C,
-    every host thread) on the same workload.  A bench step is the whole
-    workload (all its leapfrog steps) when that takes at most
-    ``JXF_REF_STEP_SECONDS`` (default 12 s) on this host, else the longest
-    prefix that fits; ``value`` is the cell updates of all timed steps over
-    their total time."""
-    if rank != 0:
-        return
-    if args.workload in ("c4", "c5"):
-        print(json.dumps({"impl": "reference", "unavailable": "the reference has neither an "
-                          "FDTD gradient nor a learned boundary or batched grids; its CPU Yee "
-                          "path is timed under the c1/c2/c3 workloads"}), flush=True)
-        return
-    n, nsteps, pml, wname = WORKLOADS[args.workload]
-    budget = float(os.environ.get("JXF_REF_STEP_SECONDS", "12"))
-    probe = cpu_baseline(args.workload, steps=4)
-    per_step = probe["seconds"] / 4
-    sample = max(4, min(nsteps, int(budget / max(per_step, 1e-9))))
-    for _ in range(args.warmup):
-        cpu_baseline(args.workload, steps=2)
-    times, updates = [], 0
-    res = None
-    for _ in range(args.steps):
-        res = cpu_baseline(args.workload, steps=sample)
-        times.append(res["seconds"])
-        updates += n ** 3 * sample
-    value = round(updates / sum(times) / 1e9, 4)
-    line = {
-        "metric": "FDTD3D Gcell-updates/s",
-        "value": value,
-        "unit": "Gcell/s",
-        "n_gpus": world,
-        "steps": args.steps,
-        "warmup": args.warmup,
-        "ms_per_step": round(1e3 * statistics.mean(times), 3),
-        "higher_is_better": True,
-        "scaling": "weak",
-        "vs_baseline": None,
-        "dtype": "f64",
-        "data": "synthetic (seeded eps_r map, pulsed dipole, seeded probes)",
-        "config": {"workload": wname, "cells": n ** 3, "leapfrog_steps_per_step": sample,
-                   "boundary": "cpml", "pml_layers": pml,
-                   "same_config": sample == nsteps},
-        "impl": "reference",
-        "cpu_baseline": {"value": value, "unit": "Gcell/s", "cores": res["cores"], "kind": "port",
-                         "sample": res["sample"]},
-        "e2e": {"value": value, "unit": "Gcell/s", "h2d_bytes_per_step": 0,
-                "d2h_bytes_per_step": 0},
-    }
-    print(json.dumps(line), flush=True)
+def run_reference(rank):
+    """The reference arm: the unmodified reference through its own API, which
+    runs on JAX; JAX is not installed and cannot be here.  (Its step restated
+    in C on the host cores is the ``cpu_baseline`` of the other arm's line.)"""
+    if rank == 0:
+        print(json.dumps({"impl": "reference",
+                          "unavailable": "the reference runs on JAX (jax, jaxlib), which is not "
+                                         "installed here and cannot be without a network"}),
+              flush=True)
 
 
 def secondary(args, world, rank, local, pg):
@@ -781,7 +739,7 @@ def main():
     world, rank, local, pg = dist_setup()
     try:
         if args.impl == "reference":
-            run_reference(args, world, rank)
+            run_reference(rank)
         elif args.workload == "c5":
             run_batch(args, world, rank, local, pg)
         elif args.workload == "c4":

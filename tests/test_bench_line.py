@@ -22,3 +22,12 @@ def test_step_roofline(n, pml, eps, in_place, bound, fields):
 
     got = bench.step_roofline(n, pml, eps, in_place)
     assert got == (bound, fields + bench.psi_bytes_per_cell(n, pml))
+
+
+def test_reference_arm_reports_itself_unavailable():
+    """It runs the reference or nothing: never this repository's own restatement."""
+    out = subprocess.run([sys.executable, str(ROOT / "bench.py"), "--impl", "reference", "--steps",
+                          "1", "--warmup", "3"], capture_output=True, text=True, check=True,
+                         timeout=300).stdout
+    line = json.loads(out)
+    assert line["impl"] == "reference" and "JAX" in line["unavailable"] and "value" not in line
