@@ -51,8 +51,9 @@ extern "C" {
 #define JXF_BND_REFLECTING 4
 
 /* Kernel path selection for 3D grids. */
-#define JXF_PATH_AUTO 0      /* TMA path when the shape allows it          */
-#define JXF_PATH_GENERIC 1   /* plain-load kernels: every mode and shape   */
+#define JXF_PATH_AUTO 0      /* the fastest: in-place passes, or the TMA   */
+                             /* path's launches where the shape allows     */
+#define JXF_PATH_GENERIC 1   /* per-cell kernels: every mode and shape     */
 #define JXF_PATH_TMA 2       /* TMA-staged marching kernel (nz % 4 == 0,   */
                              /* boundary != PERIODIC)                       */
 
@@ -154,7 +155,11 @@ int jxf_grid3d_set_probes(jxf_grid3d* g, int32_t n, const int64_t* cell,
  * (fdtd3d.py:280-393).  probe_out: DEVICE float32 [n_steps][n_probes] or
  * NULL.  Returns JXF_ERR_TIMEOUT if a bounded device wait gave up (checked
  * only when the call synchronises; see jxf_grid3d_check_error).  An x-slab
- * (jxf_grid3d_create_slab) takes it only on the TMA path, one step per call. */
+ * (jxf_grid3d_create_slab) takes it only on the TMA path, one step per call.
+ * The first step of a TMA-path grid of 2^18 cells or more times launch shapes
+ * and synchronises; after jxf_grid3d_set_sources or set_probes, the next step
+ * of a TMA-path grid may allocate.  Steps of other grids do neither, the first
+ * included, and can be captured into a CUDA graph. */
 int jxf_grid3d_step(jxf_grid3d* g, int32_t n_steps, float* probe_out, void* stream);
 
 /* Advance n_steps and keep the states after steps 1, 1 + save_every,
@@ -228,12 +233,20 @@ int jxf_grid3d_plane(jxf_grid3d* g, int32_t comp, int32_t plane, float* buf, int
                      void* stream);
 
 /* Batches of independent grids (extension; the reference runs one grid per
- * simulate() call).  jxf_batch3d_create groups existing grids (generic path,
- * same boundary mode and device; sizes may differ); they keep their own
+ * simulate() call).  jxf_batch3d_create groups existing grids (one kernel
+ * path, boundary mode and device; sizes may differ); they keep their own
  * materials, sources, probes and field access.  jxf_batch3d_step advances
- * every grid by n_steps with one kernel per phase for the whole batch; with
- * use_graph != 0 the n-step sequence is captured once into a CUDA graph
- * (cached per start step and length) and replayed with one launch.  Probe
+ * every grid by n_steps, in one of two ways that the first run of the batch
+ * chooses where every grid has desc.path JXF_PATH_AUTO (TMA-path grids: by
+ * timing both; others: by a rule on sizes and counts):
+ *   groups    up to eight grids that fit the L2 together run all n steps on
+ *             in-place passes, then the next group; plain launches, use_graph
+ *             has no effect;
+ *   lockstep  all grids step together, one launch per phase (TMA path: per
+ *             CPML part) for the whole batch; with use_graph != 0 the n-step
+ *             sequence is captured once into a CUDA graph (cached per start
+ *             step and length) and replayed with one launch.
+ * A first run that fails for want of memory has stepped no grid.  Probe
  * rows of the last run: jxf_batch3d_probes(b, grid, n_steps, dst) copies the
  * [n_steps][n_probes of that grid] trace into device memory. */
 typedef struct jxf_batch3d jxf_batch3d;
@@ -243,8 +256,8 @@ int jxf_batch3d_reset(jxf_batch3d* b, void* stream);
 int jxf_batch3d_step(jxf_batch3d* b, int32_t n_steps, int32_t use_graph, void* stream);
 int jxf_batch3d_probes(jxf_batch3d* b, int32_t grid, int32_t n_steps, float* dst, void* stream);
 /* Kernel launches per leapfrog step of the batch's current shape, and the
- * launch shape of a TMA batch (registry entry, x chunk, single-axis split;
- * -1 each for a generic batch).  No reference counterpart (the reference runs
+ * launch shape of a TMA batch in lockstep (registry entry, x chunk,
+ * single-axis split; -1 each otherwise).  No reference counterpart (the reference runs
  * one grid per simulate() call, fdtd3d.py:169). */
 int jxf_batch3d_kernels_per_step(const jxf_batch3d* b);
 int jxf_batch3d_launch(const jxf_batch3d* b, int32_t* out3);
@@ -373,7 +386,9 @@ int jxf_grid2d_set_waveforms(jxf_grid2d* g, int32_t n_waves, int64_t n_samples,
  * PEC except x in [gap_start, gap_end); gap_start < 0 means a solid wall. */
 int jxf_grid2d_set_walls(jxf_grid2d* g, int32_t n, const int32_t* y,
                          const int32_t* gap_start, const int32_t* gap_end);
-/* Replaces the scan over fdtd.py:304-364. */
+/* Replaces the scan over fdtd.py:304-364.  The first call of several steps
+ * allocates a second buffer set, unless its stream is being captured into a
+ * CUDA graph (or there is no room): it then takes one step per launch. */
 int jxf_grid2d_step(jxf_grid2d* g, int32_t n_steps, void* stream);
 /* Advance n_steps and keep the states after steps 1, 1 + save_every,
  * 1 + 2 save_every, ... (n_frames of them, all within n_steps; the frames the

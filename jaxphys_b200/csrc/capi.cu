@@ -3343,8 +3343,9 @@ namespace {
 // the steps of a call before the next group starts, and its fields cross DRAM
 // once per call instead of once per step.  64 grids of sides 68 to 180, 10-layer
 // CPML: 1.84 ms a step against 3.64 in lockstep at its best launch shape; 7
-// grids of sides 63 to 73: 45 us against 146; 64 grids behind the learned band:
-// 2.4 ms against 2.5 (the band's network is 1.0 ms of either).
+// grids of sides 63 to 73, odd ones among them: 60 us against 109; 64 grids
+// behind the learned band: 2.4 ms against 2.5 (the band's network is 1.0 ms of
+// either).  Many small grids are better off in lockstep (batch_sweep_pays).
 
 bool batch_can_sweep(const jxf_batch3d* b) {
   for (const jxf_grid3d* g : b->grids)

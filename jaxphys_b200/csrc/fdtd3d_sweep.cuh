@@ -13,7 +13,7 @@
 // 126 MB L2 from step to step, while the marching kernel's two sets do not
 // fit, and its march is a serial chain of planes with a barrier in each.  Here
 // every load of a thread is in flight at once and there is no barrier.  What
-// bounds the passes is the L1 of each SM (0.65 busy in a profiled 128^3 CPML
+// bounds the passes is the L1 of each SM (0.67 busy in a profiled 128^3 CPML
 // pass of 17.7 us that takes 12.2 unprofiled) and the wait for its loads, at
 // 66 and 73 bytes per cell, 12 TB/s, in the two passes; below 64^3 the two
 // launches of a step (about 2.4 us each).  Measured per step on one B200,

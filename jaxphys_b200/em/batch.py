@@ -5,8 +5,10 @@ boundary mode, all on one kernel path, and advances all of them together (C
 ABI ``jxf_batch3d_*``):
 
 * in-place passes (every grid ``path="auto"``; chosen on the first run where
-  they are faster): groups of grids that stay in the L2 cache, each running
-  all its steps before the next group begins.
+  they are faster: by timing on the TMA path, else by a rule on sizes and
+  counts, which leaves many small grids in lockstep): groups of grids that
+  stay in the L2 cache, each running all its steps before the next group
+  begins.  Plain launches, with or without ``use_graph``.
 * TMA path (nz % 4 == 0; ``path="auto"`` or ``"tma"``): one persistent launch
   per step (and per CPML part) over a work list of every grid's
   (tile, x-chunk) blocks, heaviest first; blocks take work through an atomic
@@ -17,8 +19,8 @@ ABI ``jxf_batch3d_*``):
   shape, odd nz included).
 
 ``run(n)`` of the last two captures the n-step sequence once into a CUDA graph
-and replays it with a single launch.  Each grid keeps its own permittivity, sources, probes
-and field accessors.  Typical use: many design candidates, or many source
+and replays it with a single launch.  Each grid keeps its own permittivity,
+sources, probes and field accessors.  Typical use: many design candidates, or many source
 positions, of one device.
 """
 

@@ -143,7 +143,9 @@ class EMGrid3D:
         pml_layers: Number of damping / CPML layers.
         cpml: CPML grading (boundary="cpml").
         device: CUDA device ordinal (default: torch's current device).
-        path: "auto", "tma" or "generic" kernel path.
+        path: "auto" (the fastest kernels for the grid), "tma" (marching and
+            blocked launches; nz % 4 == 0, not periodic) or "generic" (one
+            kernel per phase and cell, any grid: the slow reference path).
         band: boundary="learned": the ``LearnedBand`` to use (default: the
             shipped weights).
     """
