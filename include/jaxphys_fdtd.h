@@ -179,9 +179,9 @@ int jxf_grid3d_run(jxf_grid3d* g, int32_t n_steps, int32_t save_every, int64_t n
  * into probe_out (device [n_steps][n_probes], may be NULL) and keeping a
  * checkpoint of the full state every checkpoint_every steps (<= 0: the H and
  * psi_E snapshots of as many last steps as fit a sixteenth of the device's
- * memory, over all grids of the process, and an eighth of what is free beside
- * the gradient's other buffers are kept, and the steps before them get
- * checkpoints every ceil(sqrt) of their number).  The buffers stay with the
+ * memory (a quarter over all grids of the process) and an eighth of what is
+ * free beside the gradient's other buffers are kept, and the steps before them
+ * get checkpoints every ceil(sqrt) of their number).  The buffers stay with the
  * grid for its next gradient.
  * jxf_grid3d_adjoint_backward: probe_grad = dJ/d(probe_out) (device
  * [n_steps][n_probes]); writes dJ/d(eps_r) (device float32 [nx*ny*nz]).

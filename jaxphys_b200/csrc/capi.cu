@@ -4641,9 +4641,10 @@ extern "C" int jxf_grid3d_adjoint_forward(jxf_grid3d* g, int32_t n_steps,
   for (int k = 0; k < PSI_COUNT; ++k) state += psi_size(g, k);
   if (g->path == JXF_PATH_TMA) TRY(ensure_tma_ready(g, st));
   // Where the caller leaves the memory to the library, the snapshots of as
-  // many last steps as fit a sixteenth of the device (over all grids of the
-  // process, so that many of them leave a caller the rest; and an eighth of what
-  // is free) are kept, and only the steps before them are recomputed: a
+  // many last steps as fit a sixteenth of the device (and an eighth of what is
+  // free; a quarter of the device over all grids of the process, so that many
+  // of them leave a caller the rest: six of 96^3 held 76 GB without that bound)
+  // are kept, and only the steps before them are recomputed: a
   // recomputed step costs as much as a forward one (96^3, 2000 steps, 650 of
   // them kept in 11 GB: 104.8 ms a gradient against 116.7; 48^3, 300 steps, all
   // kept: 5.96 against 8.60).
@@ -4668,7 +4669,7 @@ extern "C" int jxf_grid3d_adjoint_forward(jxf_grid3d* g, int32_t n_steps,
       std::lock_guard<std::mutex> lk(g_kept.mu);
       size_t& kept = g_kept.on[g->d.device];
       kept -= 4 * g->adj_kp_cap;  // (of other grids)
-      const size_t room = total_b / 16 > kept ? total_b / 16 - kept : 0;
+      const size_t room = std::min(total_b / 16, total_b / 4 > kept ? total_b / 4 - kept : 0);
       const size_t may = std::min(room, (free_b > rest ? free_b - rest : 0) / 8) / 4;
       const size_t get = std::min(want, may / snap * snap);
       if (get > g->adj_kp_cap &&

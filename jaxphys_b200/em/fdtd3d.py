@@ -482,8 +482,8 @@ class EMGrid3D:
         """Extension: reset, run ``n_steps`` keeping what
         :meth:`adjoint_backward` needs: a checkpoint every ``checkpoint_every``
         steps, or by default the snapshots of as many last steps as fit a
-        sixteenth of the device (over all grids of the process) and sqrt(T)
-        checkpoints of the others; returns the probe traces (n_steps, P).
+        sixteenth of the device (a quarter over all grids of the process) and
+        sqrt(T) checkpoints of the others; returns the probe traces (n_steps, P).
         The memory stays with the grid: :meth:`adjoint_release`."""
         import torch
 
