@@ -342,8 +342,12 @@ __device__ __forceinline__ void sweep_block(const Step3D& p, const SweepPlan& s,
   // until this step's E pass, its H components were recorded by its E pass.
   // Spread over the planes: one block for all of them took 150 us a step for
   // 16,384 probes (33^3 CPML: 6.2 us a step with one probe); over all blocks,
-  // the test in every block costs 1.5 % of a 128^3 CPML step.
-  if (p.probe_out != nullptr && b == 0) {
+  // the test in every block costs 1.5 % of a 128^3 CPML step.  (With the whole
+  // test up front and the loop not unrolled, the kernels keep the registers
+  // they have without it: two more cost the one-cell CPML kernels a block per
+  // SM, 155 against 140 us a step for 60,000 x 8 x 9 cells.)
+  if (p.probe_out != nullptr && b == 0 && x * NT < p.n_probes) {
+#pragma unroll 1
     for (int i = x * NT + (int)threadIdx.x; i < p.n_probes; i += p.nx * NT) {
       const int c = p.probe_comp[i];
       if ((c < 3) == H) p.probe_out[i] = p.in[c][p.probe_cell[i]];
